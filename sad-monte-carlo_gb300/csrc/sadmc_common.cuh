@@ -37,6 +37,44 @@ __device__ __forceinline__ bool finite64(double x) {
   return (__double_as_longlong(x) & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
 }
 
+// Two binary32 values in one 64-bit register, for the packed operations: each half is rounded
+// as the scalar operation rounds it, at half the instructions.
+struct F32x2 { unsigned long long v; };
+__device__ __forceinline__ F32x2 f2_pack(float a, float b) {
+  F32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(F32x2 x, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F32x2 f2_add(F32x2 a, F32x2 b) {
+  F32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+// a b + z in one rounding; with z the pair of negative zeros a product.  The assembler contracts
+// a packed multiplication into the addition that uses it, whatever its rounding modifier,
+// and sees through a constant z: z comes from the launch (kNegZero2 as a kernel argument),
+// so that products and sums round separately, as the scalar operations do.
+__device__ __forceinline__ F32x2 f2_mul(F32x2 a, F32x2 b, F32x2 z) {
+  F32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(z.v));
+  return r;
+}
+__device__ __forceinline__ F32x2 f2_fma(F32x2 a, F32x2 b, F32x2 c) {
+  F32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+// 1 / x by the hardware reciprocal, the value __fdividef(1, x) has for normal x up to 2^126;
+// infinite for a zero or subnormal x.
+__device__ __forceinline__ float rcp_hw(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 template <int LPW>
 __device__ __forceinline__ unsigned group_mask(int group) {
   return LPW == 32 ? 0xffffffffu : (((1u << LPW) - 1u) << (group * LPW));

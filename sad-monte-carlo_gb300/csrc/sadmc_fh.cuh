@@ -151,12 +151,22 @@ __device__ __forceinline__ double sad_gamma_value(double p, uint64_t tF, uint64_
 // in each walker's state (WL and 1/t-WL, whose walkers switch to SAMC at run time).
 constexpr int FAM_ANY = -1;
 
-// SPLIT: the bookkeeping that no decision reads -- the acceptance rate and translation
-// scale, the energy sums, and the max-entropy / round-trip stamps -- is left to another
-// warp, which replays it from a per-move record (out_li, out_i1l, tsc_event and the
-// state after the move); this object then holds neither those fields nor their planes.
-template <int LPW, int FAM = FAM_ANY, bool SPLIT = false>
+// MODE: how the bookkeeping is divided.
+//  BOOK_FULL   everything here;
+//  BOOK_SPLIT  the bookkeeping that no decision reads -- the acceptance rate and translation
+//              scale, the energy sums, and the max-entropy / round-trip stamps -- is left to
+//              another warp, which replays it from a per-move record (out_li, out_i1l,
+//              tsc_event and the state after the move); this object then holds neither
+//              those fields nor their planes;
+//  BOOK_LEAN   everything, with an ordinary move on the lean path (lean_decide, lean_finish).
+//              The energy sums are atomic additions that nothing waits for (one lane's
+//              additions to one address keep their order, so the sums round as sequential
+//              ones), and t_found is written where it is set instead of being cached.
+constexpr int BOOK_FULL = 0, BOOK_SPLIT = 1, BOOK_LEAN = 2;
+template <int LPW, int FAM = FAM_ANY, int MODE = BOOK_FULL>
 struct Fh {
+  static constexpr bool SPLIT = MODE == BOOK_SPLIT, LEAN = MODE == BOOK_LEAN;
+  static constexpr bool SUMS = MODE == BOOK_FULL;  // the energy sums are cached here
   static_assert(!SPLIT || (LPW == 1 && FAM == M_SAD), "the split bookkeeping is SAD on one lane");
   WalkerCore c;
   // launch constants
@@ -212,6 +222,20 @@ struct Fh {
   bool tsc_event;
   __device__ void invalidate_gamma() { gb_ok = 0; xg_ok = false; ++pgen; }
   bool inverted;        // too_lo > too_hi (never true for SAD; kept exact)
+  // LEAN: binary32 views of the state for lean_decide (lean_sync refreshes them after the
+  // generic bookkeeping, lean_finish after an ordinary move)
+  int cls, cls2;        // -1 / 0 / +1: E (the proposed energy) below / inside / above the SAD window
+  float kf, a1f, ea;    // k_lnw; ln w the Metropolis test uses at E and its error bound
+  float maxSf, ddB;     // max_S; the error bound of a difference of two weights
+  // Thresholds of the proposed energy's binary32 estimate, each moved by the estimate's error
+  // bound: surely inside the allocated bins and the allowed energies; surely above / below
+  // the allowed energies; surely inside / above / below the SAD window
+  float in_lo, in_hi, out_hi, out_lo, tinyB, win_in_lo, win_in_hi, win_out_lo, win_out_hi;
+  float binB;           // distance from a bin edge, in bins, within which the estimate may err
+  float tlof, invTf, lwlo, lwhi, belowB;  // too_lo, 1/min_T, ln w of the window's edge bins
+  int lw_lo, lw_hi;     // the bins lwlo and lwhi were taken from
+  bool lean_off;        // every move takes the generic bookkeeping
+  double* gtab;         // this walker's 4 LPW gammas in shared memory (LPW > 1)
 
   // ---- index helpers ---------------------------------------------------------------
   __device__ int gidx_exact(double e) const { return (int)((e - c.cur_min) / width) + c.b_lo; }
@@ -233,29 +257,36 @@ struct Fh {
   // cached-bin aware accessors
   __device__ double ld_lnw(int g) const { return g == cur ? k_lnw : lnw[g]; }
   __device__ uint64_t ld_hist(int g) const { return g == cur ? k_hist : hist[g]; }
-  __device__ uint64_t ld_tf(int g) const { return g == cur ? k_tf : tf[g]; }
+  __device__ uint64_t ld_tf(int g) const { return g == cur && !LEAN ? k_tf : tf[g]; }
   __device__ void st_lnw(int g, double v) {
     if (g == cur) k_lnw = v;
     else if (wr) lnw[g] = v;
   }
   __device__ void flush_cur() {
     if (wr) {
-      lnw[cur] = k_lnw; hist[cur] = k_hist; tf[cur] = k_tf;
-      if (!SPLIT) { sE[cur] = k_sE; sE2[cur] = k_sE2; }
+      lnw[cur] = k_lnw; hist[cur] = k_hist;
+      if (!LEAN) tf[cur] = k_tf;
+      if (SUMS) { sE[cur] = k_sE; sE2[cur] = k_sE2; }
     }
   }
   __device__ void load_cur(int g) {
     g = g < 0 ? 0 : (g >= nbins ? nbins - 1 : g);
     cur = g;
-    k_lnw = lnw[g]; k_hist = hist[g]; k_tf = tf[g];
-    if (!SPLIT) { k_sE = sE[g]; k_sE2 = sE2[g]; k_stamp = stamp[g]; }
+    k_lnw = lnw[g]; k_hist = hist[g];
+    if (!LEAN) k_tf = tf[g];
+    if (SUMS) { k_sE = sE[g]; k_sE2 = sE2[g]; }
+    if (!SPLIT) k_stamp = stamp[g];
   }
   __device__ void fetch_pending(int g) {
     if (g == cur) {
-      p_lnw = k_lnw; p_hist = k_hist; p_tf = k_tf; p_sE = k_sE; p_sE2 = k_sE2; p_stamp = k_stamp;
+      p_lnw = k_lnw; p_hist = k_hist; p_stamp = k_stamp;
+      if (!LEAN) p_tf = k_tf;
+      if (SUMS) { p_sE = k_sE; p_sE2 = k_sE2; }
     } else {
-      p_lnw = lnw[g]; p_hist = hist[g]; p_tf = tf[g];
-      if (!SPLIT) { p_sE = sE[g]; p_sE2 = sE2[g]; p_stamp = stamp[g]; }
+      p_lnw = lnw[g]; p_hist = hist[g];
+      if (!LEAN) p_tf = tf[g];
+      if (SUMS) { p_sE = sE[g]; p_sE2 = sE2[g]; }
+      if (!SPLIT) p_stamp = stamp[g];
     }
   }
   // adopt the prefetched fields of bin g (== i2) as the current bin
@@ -263,8 +294,10 @@ struct Fh {
     if (g == cur) return;
     flush_cur();
     cur = g;
-    k_lnw = p_lnw; k_hist = p_hist; k_tf = p_tf;
-    if (!SPLIT) { k_sE = p_sE; k_sE2 = p_sE2; k_stamp = p_stamp; }
+    k_lnw = p_lnw; k_hist = p_hist;
+    if (!LEAN) k_tf = p_tf;
+    if (SUMS) { k_sE = p_sE; k_sE2 = p_sE2; }
+    if (!SPLIT) k_stamp = p_stamp;
   }
   __device__ void move_cur(int g) {
     if (g != cur) { flush_cur(); load_cur(g); }
@@ -328,6 +361,7 @@ struct Fh {
     inv_tF_of = 0; inv_ns_of = 0; inv_tF = inv_ns = 0.0;
     tF_d = ns_d = 0.0;
     g_zero = true;
+    lw_lo = lw_hi = -1;
     xg = nullptr;
     xg_t0 = 0;
     xg_ok = false;
@@ -399,6 +433,26 @@ struct Fh {
       return gamma_at(c.moves);
     }
     constexpr uint32_t SPAN = 4 * LPW;
+    if (LEAN && LPW > 1) {  // the batch in shared memory: one load per move
+      const int off = (int)((uint32_t)c.moves & (SPAN - 1)), qc = off / LPW;
+      if (off == 0) gb_ok = 0;
+      if (SADMC_RARE(!((gb_ok >> qc) & 1u))) {
+        if (kind() == M_SAD) refresh_sad_params();
+        const uint64_t t0 = c.moves - (uint64_t)off + (uint64_t)glane;
+        sync();
+        if (off == 0 || LPW == 32) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (q >= qc) gtab[LPW * q + glane] = gamma_at(t0 + (uint64_t)(LPW * q));
+          gb_ok = 0xfu;
+        } else {
+          gtab[LPW * qc + glane] = gamma_at(t0 + (uint64_t)(LPW * qc));
+          gb_ok |= 1u << qc;
+        }
+        sync();
+      }
+      return gtab[off];
+    }
     const uint32_t m32 = (uint32_t)c.moves;
     const uint32_t base = m32 & ~(SPAN - 1);
     const int off = (int)(m32 - base);
@@ -600,15 +654,7 @@ struct Fh {
         if (i2 <= win_lo || i2 >= win_hi) exact();  // extrapolation / edge comparisons
         const double lnw2 = sad_lnw(e2, i2);
         rejected = dgt(lnw2, lnw1) && metropolis_reject2(lnw1, lnw2, u53);
-        if (SADMC_RARE(!rejected && hist2 == 0)) {  // energy.rs:466-483
-          exact();
-          if (e2 < c.too_hi && e2 > c.too_lo) {
-            c.latest_param = div_by(c.too_hi - c.too_lo, c.min_T, inv_minT);
-            c.num_states += 1;
-            c.tL = c.moves;
-            invalidate_gamma();
-          }
-        }
+        if (SADMC_RARE(!rejected && hist2 == 0)) sad_discovery(e2);
         break;
       }
       case M_SAMC: {
@@ -631,30 +677,237 @@ struct Fh {
     return rejected;
   }
 
+  // ---- the lean path -------------------------------------------------------------------
+  // An ordinary move -- its proposed bin allocated, no threshold within the binary32
+  // estimates' error bounds, no window growth -- decided and booked in
+  // straight-line code on 32-bit quantities where those decide; every other move takes
+  // decide_de and finish_move, which the lean path leaves untouched.  On the serial chain of
+  // a walker each instruction costs about five cycles, so the number of them is what counts.
+
+  // The binary32 views from the state.  With |E|, |e2| <= B in the allocated range, the
+  // estimate e2f = Ef + de is within 2 B 2.5e-7 of e2 (see decide_de); the thresholds take
+  // 4e-7, which also covers their own rounding.
+  __device__ void lean_sync() {
+    const float B = fmaxf(fmaxf(fabsf(cminf), fabsf(cmaxf)), fabsf(Ef)), u = 4.0e-7f;
+    const float tolB = 2.0f * B * u + 1e-30f;
+    in_lo = cminf + (tolB + fabsf(cminf) * u);
+    in_hi = cmaxf - (tolB + fabsf(cmaxf) * u);
+    out_hi = INFINITY; out_lo = -INFINITY;
+    if (has_max_allowed) {
+      in_hi = fminf(in_hi, maxf - (tolB + fabsf(maxf) * u));
+      out_hi = maxf + (tolB + 3.0f * fabsf(maxf) * u);
+    }
+    if (has_min_allowed) {
+      in_lo = fmaxf(in_lo, minf + (tolB + fabsf(minf) * u));
+      out_lo = minf - (tolB + 3.0f * fabsf(minf) * u);
+    }
+    tinyB = B * 1e-15f + 1e-37f;
+    binB = (tolB + fabsf(cminf) * u) * inv_wf + fabsf((cmaxf - cminf) * inv_wf) * u + 1e-6f;
+    kf = lean_f32(k_lnw);
+    maxSf = f32_trunc(c.max_S);
+    ddB = fabsf(maxSf) * 6.0e-7f + 1e-30f;
+    cls = 0;
+    lean_off = (kind() != M_SAD && kind() != M_SAMC && kind() != M_WL) || binB > 0.25f || !(ddB < 0.2f) ||
+               (float)(c.b_hi - c.b_lo) > 4.0e6f;
+    if (kind() == M_SAD) {
+      lean_off = lean_off || inverted;
+      const float thif = f32_trunc(c.too_hi);
+      tlof = f32_trunc(c.too_lo);
+      const float ml = tolB + fabsf(tlof) * u, mh = tolB + fabsf(thif) * u;
+      win_in_lo = tlof + ml; win_out_lo = tlof - ml;
+      win_in_hi = thif - mh; win_out_hi = thif + mh;
+      invTf = (float)inv_minT;
+      belowB = ml * invTf * 1.01f;
+      if (cur == win_lo) lwlo = kf;
+      else if (lw_lo != win_lo) lwlo = lean_f32(lnw[win_lo]);
+      if (cur == win_hi) lwhi = kf;
+      else if (lw_hi != win_hi) lwhi = lean_f32(lnw[win_hi]);
+      lw_lo = win_lo; lw_hi = win_hi;
+      cls = below(c.E, cur) ? -1 : (above(c.E, cur) ? 1 : 0);
+    }
+    lean_a1();
+  }
+  // ln w truncated to binary32 for 0 and [2^-126, 2^127): (double's bits >> 29) with the
+  // exponent rebased, a smaller value as 0; a negative, huge or NaN weight gives NaN, which
+  // leaves the Metropolis test undecided.
+  __device__ static float lean_f32(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned f = __funnelshift_l(lo, hi, 3) ^ 0x40000000u;
+    const unsigned v = hi < 0x38100000u ? 0u : (f & 0x7fffffffu);
+    return __uint_as_float(hi < 0x47e00000u ? v : 0x7fc00000u);
+  }
+  // (double)f for zero and normal f, by integer instructions
+  __device__ static double lean_f64(float f) {
+    const unsigned b = __float_as_uint(f), a = b & 0x7fffffffu, sign = b & 0x80000000u;
+    const unsigned hi = a == 0u ? sign : (((a >> 3) + 0x38000000u) | sign);  // f normal or 0
+    return __hiloint2double((int)hi, (int)(b << 29));
+  }
+  // The extrapolation below too_lo with slope 1/min_T (energy.rs:461-462) at the binary32
+  // energy ef, and its error bound.
+  __device__ float lean_below(float ef, float& err) const {
+    const float x = (ef - tlof) * invTf;
+    err = __fmaf_rn(fabsf(x) + fabsf(lwlo), 4.0e-7f, belowB);
+    return lwlo + x;
+  }
+  __device__ void lean_a1() {
+    a1f = kf;
+    ea = ddB;
+    if (kind() == M_SAD && cls != 0) {
+      a1f = lwhi;
+      if (cls < 0) { a1f = lean_below(Ef, ea); ea += ddB; }
+    }
+  }
+  // 1 accepted, 0 rejected, 2: the move is for decide_de.  Everything decide_de decides on e2
+  // is taken here from e2f = Ef + de against the moved thresholds; the Metropolis test from
+  // the binary32 weights a, b with |(a - b) - (lnw1 - lnw2)| <= dd (see metropolis_reject2).
+  // The proposed bin's fields are left in p_*.
+  __device__ int lean_decide(bool possible, float de, uint64_t u53) {
+    const float e2f = Ef + de;
+    const bool ordinary = e2f > in_lo && e2f < in_hi;
+    const bool oob = (e2f > out_hi && de > tinyB) || (e2f < out_lo && de < -tinyB);
+    // the bin: nearest integer of q by adding 1.5 2^23 (|q| < 2^22), then the floor
+    const float q = (e2f - cminf) * inv_wf;
+    const float qm = q + 12582912.0f, fr = q - (qm - 12582912.0f);
+    const int qi = __float_as_int(qm) - 0x4B400000 - (fr < 0.0f ? 1 : 0);
+    const bool edge = !(fabsf(fr) > binB);
+    // clamped into the allocated range, so that the loads stay inside it
+    i2 = c.b_lo + min(max(qi, 0), c.b_hi - c.b_lo);
+    p_lnw = lnw[i2]; p_hist = hist[i2]; p_stamp = stamp[i2];
+    float b2f = i2 == cur ? kf : lean_f32(p_lnw);
+    float dd = ea;
+    cls2 = 0;
+    if (kind() == M_SAD && !(e2f > win_in_lo && e2f < win_in_hi)) {
+      cls2 = e2f < win_out_lo ? -1 : (e2f > win_out_hi ? 1 : 0);
+      if (SADMC_RARE(cls2 == 0)) {  // within the bound of an edge: the FP64 comparisons
+        const double e2 = c.E + f2d(de);
+        cls2 = e2 < c.too_lo ? -1 : (e2 > c.too_hi ? 1 : 0);
+      }
+      if (cls2 > 0) b2f = lwhi;
+      if (cls2 < 0) { float eb; b2f = lean_below(e2f, eb); dd += eb; }
+    }
+    const float df = a1f - b2f;
+    const float e32 = __expf(df);
+    const float mt = __fmaf_rn(fabsf(df), 6.0e-7f, __fmaf_rn(dd, 2.0f, 4.0e-6f));
+    const float uf = (float)(uint32_t)(u53 >> 29) * (1.0f / 16777216.0f);  // u in [uf, uf + 2^-24)
+    const bool rej = uf > __fmaf_rn(e32, mt, e32), acc = uf + (1.0f / 16777216.0f) < __fmaf_rn(-e32, mt, e32);
+    const bool small = fabsf(de) <= tinyB && de != 0.0f;  // binary32 subnormals among them
+    const bool decided = oob || (ordinary && !edge && !small && dd < 0.25f && (acc || rej));
+    if (SADMC_RARE(lean_off)) return 2;
+    if (!possible || !(fabsf(de) <= 3.0e38f)) return 0;
+    return decided ? (acc && !oob ? 1 : 0) : 2;
+  }
+  // An accepted lean move: the counters and the state of the proposed bin.
+  __device__ void lean_accept(float de, double rs) {
+    c.accepted += 1;
+    c.acc_rate += rs;
+    c.E += lean_f64(de);
+    E2 = c.E * c.E;
+    Ef = f32_trunc(c.E);
+    if (i2 != cur) {
+      flush_cur();
+      cur = i2;
+      k_lnw = p_lnw; k_hist = p_hist; k_stamp = p_stamp;
+      kf = lean_f32(k_lnw);
+    }
+    cls = cls2;
+    if (SADMC_RARE(k_hist == 0)) {  // a first visit
+      if (kind() == M_SAD) sad_discovery(c.E);
+      else if (kind() == M_WL && c.lowest_hist > 0) c.wl_num_states += 1.0;
+    }
+  }
+  // Histogram, sums, update_weights and max-entropy bookkeeping of a move that the lean path
+  // decided (energy.rs:934-965); old_cur the bin before it.
+  __device__ void lean_finish(int old_cur) {
+    if (kind() == M_SAD && SADMC_RARE(cls != 0 && k_hist >= c.highest_hist)) {
+      finish_adopted(old_cur);  // the window grows
+      lean_sync();
+      return;
+    }
+    if (SADMC_RARE(k_hist == 0)) set_found();
+    k_hist += 1;
+    add_sums();
+    if (kind() == M_SAD) {
+      const double g = gamma();
+      if (SADMC_RARE(is_nan64(g))) c.status |= ST_NAN_GAMMA;
+      if (cls == 0) {
+        if (k_hist > c.highest_hist) c.highest_hist = k_hist;
+        k_lnw += g;
+        kf = lean_f32(k_lnw);
+      }
+      if (SADMC_RARE(c.tL == c.moves)) sad_new_tF();
+      if (cur == win_lo) lwlo = kf;
+      if (cur == win_hi) lwhi = kf;
+    } else {
+      update_weights(c.E);
+      kf = lean_f32(k_lnw);
+    }
+    // energy.rs:950-965; truncation keeps the order of the weights
+    const int li = cur - c.b_lo;
+    if (SADMC_RARE(!(kf < maxSf) && dgt(k_lnw, c.max_S))) {
+      c.max_S = k_lnw;
+      maxSf = kf;
+      ddB = fabsf(maxSf) * 6.0e-7f + 1e-30f;
+      if (!(ddB < 0.2f)) lean_off = true;
+      c.max_S_local = li;
+      fill_visited(true);
+    } else if (SADMC_RARE(li == c.max_S_local)) {
+      if (old_cur != cur) fill_visited(false);
+    } else if (!visited_cur()) {
+      k_stamp = c.fill_gen;
+      if (wr) { stamp[cur] = c.fill_gen; rt[cur] = rt[cur] + 1; }
+    }
+    lean_a1();
+  }
+
+  // A bin visited for the first time, at energy e2 (energy.rs:466-483)
+  __device__ void sad_discovery(double e2) {
+    if (e2 < c.too_hi && e2 > c.too_lo) {
+      c.latest_param = div_by(c.too_hi - c.too_lo, c.min_T, inv_minT);
+      c.num_states += 1;
+      c.tL = c.moves;
+      invalidate_gamma();
+    }
+  }
+  // The first visit's move count (energy.rs:938-940)
+  __device__ void set_found() {
+    if (LEAN) { if (wr) tf[cur] = c.moves; }
+    else k_tf = c.moves;
+    if (kind() == M_SAD && cur >= win_lo && cur <= win_hi && c.moves > c.win_tmax) c.win_tmax = c.moves;
+  }
+
   // Histogram, energy sums, update_weights and max-entropy bookkeeping
   // (energy.rs:934-965).  Call after the system confirmed (c.E updated) or not.
   __device__ void finish_move(bool accepted) {
     if (c.kind == M_DESCENT) return;
     int old_cur = cur;
     if (accepted) adopt_pending(i2);
+    finish_adopted(old_cur);
+  }
+  // finish_move once the accepted bin is the cached one.
+  __device__ void finish_adopted(int old_cur) {
     const double E = c.E;
-    if (SADMC_RARE(k_hist == 0)) {  // energy.rs:938-940
-      k_tf = c.moves;
-      if (kind() == M_SAD && cur >= win_lo && cur <= win_hi && c.moves > c.win_tmax) c.win_tmax = c.moves;
-    }
+    if (SADMC_RARE(k_hist == 0)) set_found();
     k_hist += 1;
-    if (!SPLIT) {
+    if (SUMS) {
       k_sE += E;
       k_sE2 += E2;  // E2 == E * E (set_E)
     }
+    if (LEAN) add_sums();
     if (SPLIT) tsc_event = false;
     update_weights(E);
-    const int li = cur - c.b_lo;
     if (SPLIT) {
-      out_li = li;
+      out_li = cur - c.b_lo;
       out_i1l = (grew_front ? gidx_exact(e1) : old_cur) - c.b_lo;
       return;
     }
+    max_entropy(old_cur);
+  }
+  __device__ void add_sums() {  // energy.rs:941-942
+    if (wr && (LPW == 1 || glane == 0)) { atomicAdd(&sE[cur], c.E); atomicAdd(&sE2[cur], E2); }
+  }
+  // energy.rs:950-965, old_cur the bin before the move
+  __device__ void max_entropy(int old_cur) {
+    const int li = cur - c.b_lo;
     if (dgt(k_lnw, c.max_S)) {
       c.max_S = k_lnw;
       c.max_S_local = li;
@@ -735,16 +988,17 @@ struct Fh {
         invalidate_gamma();
       }
     }
-    if (SADMC_RARE(c.tL == c.moves)) {
-      uint64_t old_tF = c.tF;
-      c.tF = c.win_tmax;
-      invalidate_gamma();
-      if (SPLIT) {
-        tsc_event = old_tF != c.tF && acc_mode;
-      } else if (old_tF != c.tF && acc_mode) {  // energy.rs:600-609
-        c.tscale *= rate_factor(c.acc_rate, target_rate, inv_target);
-        tscale_changed = true;
-      }
+    if (SADMC_RARE(c.tL == c.moves)) sad_new_tF();
+  }
+  __device__ void sad_new_tF() {  // energy.rs:584-621
+    uint64_t old_tF = c.tF;
+    c.tF = c.win_tmax;
+    invalidate_gamma();
+    if (SPLIT) {
+      tsc_event = old_tF != c.tF && acc_mode;
+    } else if (old_tF != c.tF && acc_mode) {  // energy.rs:600-609
+      c.tscale *= rate_factor(c.acc_rate, target_rate, inv_target);
+      tscale_changed = true;
     }
   }
 
@@ -854,6 +1108,23 @@ struct RecentScale {
     const int src = (int)off++;
     r = __shfl_sync(0xffffffffu, rs, src);
     om = __shfl_sync(0xffffffffu, omrs, src);
+  }
+};
+
+// sqrt(1/t) and 1 - sqrt(1/t) of 32 consecutive moves in a warp's shared memory: filled by
+// its 32 lanes (whose walkers share the move count), read with one load per move.
+struct RateTable {
+  double2 v[32];  // x = sqrt(1/t), y = 1 - x (energy.rs:913)
+  // the factors of the it-th move of a launch, the moves counted before it; called by the
+  // whole warp
+  __device__ double2 get(uint32_t it, uint64_t moves, int lane) {
+    if ((it & 31u) == 0) {
+      const double r = sqrt(1.0 / (double)(moves + 1 + (uint64_t)lane));
+      __syncwarp();
+      v[lane] = make_double2(r, 1. - r);
+      __syncwarp();
+    }
+    return v[it & 31u];
   }
 };
 

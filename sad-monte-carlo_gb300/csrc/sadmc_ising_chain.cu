@@ -195,7 +195,7 @@ __host__ __device__ inline size_t ising_pipe_bytes(int nbins, int L) {
          2 * 32 * (sizeof(PipeLog) + sizeof(PipeExt)) + 2 * sizeof(PipeSnap) + 2 * sizeof(uint64_t);
 }
 
-using FhSplit = Fh<1, M_SAD, true>;
+using FhSplit = Fh<1, M_SAD, BOOK_SPLIT>;
 
 // Integer view of a SAD walker: energy, bin range, window and bounds (see above).
 struct LeanSad {

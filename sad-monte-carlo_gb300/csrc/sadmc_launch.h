@@ -34,6 +34,7 @@ struct LjSys {
   float* pos;
   int np;
   double radius2;
+  unsigned long long neg_zero2 = 0x8000000080000000ull;  // two binary32 -0 (f2_mul)
 };
 cudaError_t launch_lj_move(const MoveLaunch& m, const LjSys& s, int lpw, cudaStream_t st);
 // The shared-memory LJ move kernel with one or two lanes per walker (sadmc_lj_lane.cu),

@@ -12,6 +12,36 @@ __device__ __forceinline__ float lj_v32(float r2) {  // 4 (s^6 - s^3), s = 1/r^2
   return 4.0f * s3 * (s3 - 1.0f);
 }
 
+// The spherical wall: a move to t from f is impossible iff |t|^2 > R^2 and |t|^2 > |f|^2
+// (lj.rs:87-90), on binary32 squares where they decide and FP64 ones otherwise.
+__device__ __forceinline__ bool lj_outside(DS tx, DS ty, DS tz, DS fx, DS fy, DS fz, float R2, double radius2) {
+  const float r2t = tx.h * tx.h + ty.h * ty.h + tz.h * tz.h;
+  const float r2f = fx.h * fx.h + fy.h * fy.h + fz.h * fz.h;
+  const bool in = r2t < R2 * (1.0f - 1e-5f);
+  const bool out = r2t > R2 * (1.0f + 1e-5f) && r2t > r2f * (1.0f + 1e-5f);
+  if (!SADMC_RARE(!(in || out))) return out;
+  const double a = ds_to_double(tx), b = ds_to_double(ty), c = ds_to_double(tz);
+  const double p = ds_to_double(fx), q = ds_to_double(fy), r = ds_to_double(fz);
+  const double nt = a * a + b * b + c * c, nf = p * p + q * q + r * r;
+  return nt > radius2 && nt > nf;
+}
+
+// lj_v32 of two pairs at once: d = (ph - qh) + (pl - ql) on each axis for two atoms p
+// against one point q given as its negated double-single parts.  (A pair closer than 2^-63
+// overflows either way.)
+__device__ __forceinline__ F32x2 lj_v32x2(const F32x2 ph[3], const F32x2 pl[3], const F32x2 nh[3],
+                                          const F32x2 nl[3], F32x2 z) {
+  F32x2 d[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) d[c] = f2_add(f2_add(ph[c], nh[c]), f2_add(pl[c], nl[c]));
+  const F32x2 r2 = f2_add(f2_add(f2_mul(d[0], d[0], z), f2_mul(d[1], d[1], z)), f2_mul(d[2], d[2], z));
+  float a, b;
+  f2_unpack(r2, a, b);
+  const F32x2 sv = f2_pack(rcp_hw(a), rcp_hw(b));
+  const F32x2 s3 = f2_mul(f2_mul(sv, sv, z), sv, z);
+  return f2_mul(f2_mul(f2_pack(4.0f, 4.0f), s3, z), f2_add(s3, f2_pack(-1.0f, -1.0f)), z);
+}
+
 template <int LPW, int APL>
 struct LjWalker {
   DS x[APL], y[APL], z[APL];
@@ -70,21 +100,7 @@ struct LjWalker {
     tx = ds_add(fx, ds_scale(g0, sh, sl));
     ty = ds_add(fy, ds_scale(g1, sh, sl));
     tz = ds_add(fz, ds_scale(g2, sh, sl));
-    // wall: impossible iff |to|^2 > R^2 and |to|^2 > |from|^2 (lj.rs:87-90)
-    const float r2t = tx.h * tx.h + ty.h * ty.h + tz.h * tz.h;
-    const float r2f = fx.h * fx.h + fy.h * fy.h + fz.h * fz.h;
-    const float R2 = wall_r2f;
-    bool impossible;
-    if (r2t < R2 * (1.0f - 1e-5f)) {
-      impossible = false;
-    } else if (r2t > R2 * (1.0f + 1e-5f) && r2t > r2f * (1.0f + 1e-5f)) {
-      impossible = true;
-    } else {
-      double a = ds_to_double(tx), b = ds_to_double(ty), c = ds_to_double(tz);
-      double p = ds_to_double(fx), q = ds_to_double(fy), r = ds_to_double(fz);
-      double nt = a * a + b * b + c * c, nf = p * p + q * q + r * r;
-      impossible = nt > radius2 && nt > nf;
-    }
+    const bool impossible = lj_outside(tx, ty, tz, fx, fy, fz, wall_r2f, radius2);
     if (impossible) return false;
     float de = 0.0f;
     // Differences of double-single positions: the high parts of two nearby atoms subtract

@@ -1,0 +1,76 @@
+"""The lean path of the bookkeeping (an ordinary move decided on binary32 thresholds) against
+the FP64 oracle, where its thresholds matter: bins too narrow for it, energy bounds on either
+side or none, every method, ragged batches and launches that end inside a table batch."""
+import numpy as np
+import pytest
+
+from helpers import METHOD_KW, assert_bins_equal, assert_scalars_equal, ising_spins, lj_configs
+
+pytestmark = pytest.mark.gpu
+
+REPLAY_REL = 2e-5  # binary32 pair energies against FP64 ones, see test_gpu_lj.py
+
+
+@pytest.mark.parametrize("lanes", [8, 2, 1])
+@pytest.mark.parametrize("kw", [
+    dict(method="sad", energy_bin=0.0001, min_allowed=-11.0, max_allowed=-10.0, e_lo=-13.0,
+         e_hi=-8.0),                                                   # narrower than the estimate's error
+    dict(method="sad", energy_bin=0.5, min_allowed=-25.0, max_allowed=-8.0),
+    dict(method="sad", energy_bin=0.2, max_allowed=None, e_hi=400.0),  # no upper bound: proposals out of range
+    dict(method="samc", energy_bin=0.2),
+    dict(method="wl", energy_bin=2.0),
+    dict(method="inv_t_wl", energy_bin=4.0),
+    dict(method="canonical", energy_bin=0.2),
+], ids=lambda k: f"{k['method']}-{k['energy_bin']}")
+def test_lj_lean_path(gpu, oracle, kw, lanes):
+    n, W, radius, seed, runs = 13, 5, 2.2, 11, (1200, 37, 500)
+    okw = dict(METHOD_KW[kw["method"]], energy_bin=kw["energy_bin"], target_rate=0.5, translation_scale=0.1,
+               max_allowed=kw.get("max_allowed", 0.0), min_allowed=kw.get("min_allowed"))
+    okw = {k: v for k, v in okw.items() if v is not None}
+    confs = lj_configs(oracle, n, radius, range(40, 40 + W))
+    b = gpu.Batch(gpu.make_config(gpu.LJ, W, n, e_lo=kw.get("e_lo", -50.0), e_hi=kw.get("e_hi", 5.0), seed=seed,
+                                  lanes_per_walker=lanes, **okw), [(n, radius, (0, 0, 0))] * W)
+    b.upload(confs)
+    b.initialize()
+    E0 = b.energies()
+    moves = sum(runs)
+    b.set_trace(moves)
+    for k in runs:
+        b.run(k)
+    out_of_range = b.status() & gpu.ST_BIN_RANGE
+    for w in (0, 3, W - 1):
+        if out_of_range[w]:
+            continue  # the reference would have grown its bins
+        e1, e2 = b.trace(w, moves)
+        ow = oracle.Walker(oracle.make_config(oracle.LJ, n, radius=radius, seed=seed, walker=w, e0=float(E0[w]),
+                                              **okw), confs[w])
+        disc, mismatch = ow.run_override(e1, e2)
+        assert mismatch == 0 and disc < REPLAY_REL, (w, mismatch, disc)
+        assert_bins_equal(b.bins(w), ow.bins(), label=f"walker {w}")
+        assert_scalars_equal(b.scalars(w), ow.scalars(), label=f"walker {w}")
+        np.testing.assert_allclose(b.state(w), ow.state(), atol=1e-11)
+
+
+@pytest.mark.parametrize("method,energy_bin,bounds", [
+    ("sad", 1.0, None), ("sad", 3.0, (-300.0, 250.0)), ("sad", 0.25, (-60.0, 60.0)), ("samc", 8.0, (-400.0, None)),
+    ("wl", 16.0, None), ("inv_t_wl", 16.0, (-450.0, 100.0)), ("canonical", 4.0, None)])
+def test_ising_lean_path_bit_exact(gpu, oracle, method, energy_bin, bounds):
+    L, W, seed = 16, 35, 13
+    N = L * L
+    kw = dict(METHOD_KW[method], energy_bin=energy_bin)
+    if bounds:
+        kw.update({k: v for k, v in zip(("min_allowed", "max_allowed"), bounds) if v is not None})
+    b = gpu.Batch(gpu.make_config(gpu.ISING, W, L, e_lo=-2.0 * N - 20, e_hi=2.0 * N + 20, seed=seed,
+                                  lanes_per_walker=1, **kw), [(L, 0.0, (0, 0, 0))] * W)
+    spins = [ising_spins(L, 500 + w) for w in range(W)]
+    b.upload(spins)
+    b.initialize()
+    for k in (7001, 33, 5000):
+        b.run(k)
+    for w in (0, 1, 31, 32, 34):
+        ow = oracle.Walker(oracle.make_config(oracle.ISING, L, seed=seed, walker=w, **kw), spins[w])
+        ow.run(12034)
+        assert_bins_equal(b.bins(w), ow.bins(), label=f"walker {w}")
+        assert_scalars_equal(b.scalars(w), ow.scalars(), label=f"walker {w}")
+        np.testing.assert_array_equal(b.state(w), ow.state())
+    assert not b.status().any()
