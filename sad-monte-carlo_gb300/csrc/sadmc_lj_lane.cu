@@ -7,12 +7,13 @@
 // shuffles at all.  The pair work, 2 (N-1) binary32 terms, runs in the walker's own lane
 // (or two), at full FP32 rate.
 //
-// Layout: each warp holds its walkers' double-single positions (hi, lo as a float2) in
-// shared memory as [coordinate][atom slot][walker of the warp][lane of the walker], atom
-// j = lane + LPW * slot, so that the 32 lanes of a warp reading "their" atom of one slot
-// touch 32 consecutive 8-byte words (two wavefronts of 16 lanes, no bank conflict; with
-// the lanes of a walker 16 walkers apart instead, a wavefront's two halves met the same
-// banks).
+// Layout: each warp holds its walkers' double-single positions in shared memory as
+// [coordinate][high, low][slot pair][lane], atom j = lane + LPW * slot: a lane reads two of
+// its atoms' values with one 64-bit load (conflict-free) for the packed pair terms, which
+// take two atoms per instruction.  Draws, gamma and sqrt(1/t) come from tables in shared
+// memory as in the register kernel.
+// Measured on one GB300 (8192 LJ38 walkers, 2 lanes, SAD): 8.8 -> 4.8 us per step against
+// the scalar pair terms over all 64 slots and the general bookkeeping on every move.
 // Global memory keeps the register kernel's [walker][6][np] planes, so the two kernels
 // continue each other's runs.
 #include <cuda_runtime.h>
@@ -28,183 +29,183 @@
 namespace sadmc {
 namespace dev {
 
-// 4 (s^6 - s^3), s = 1/r^2 (lj.rs:78-81) in binary32 with fused steps (the kernels'
-// pair terms carry a stated tolerance; the FP64 re-sum and the oracle replay bound it).
-__device__ __forceinline__ float lj_v32_fused(float dx, float dy, float dz) {
-  const float r2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-  const float s = __fdividef(1.0f, r2);
-  const float s3 = __fmul_rn(__fmul_rn(s, s), s);
-  return __fmul_rn(4.0f, __fmaf_rn(s3, s3, -s3));
+// 4 (s^6 - s^3), s = 1/r^2 (lj.rs:78-81) in binary32 with fused steps, of two atoms p against
+// one point given as its negated double-single parts (the kernels' pair terms carry a stated
+// tolerance; the FP64 re-sum and the oracle replay bound it).  Double-single differences: the
+// high parts of nearby atoms subtract exactly.
+__device__ __forceinline__ F32x2 lj_v32x2_fused(const F32x2 ph[3], const F32x2 pl[3], const F32x2 nh[3],
+                                                const F32x2 nl[3], F32x2 z) {
+  F32x2 d[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) d[c] = f2_add(f2_add(ph[c], nh[c]), f2_add(pl[c], nl[c]));
+  const F32x2 r2 = f2_fma(d[0], d[0], f2_fma(d[1], d[1], f2_mul(d[2], d[2], z)));
+  float a, b;
+  f2_unpack(r2, a, b);
+  const F32x2 s = f2_pack(rcp_hw(a), rcp_hw(b));
+  const F32x2 s3 = f2_mul(f2_mul(s, s, z), s, z);
+  const F32x2 n3{s3.v ^ 0x8000000080000000ull};
+  return f2_mul(f2_pack(4.0f, 4.0f), f2_fma(s3, s3, n3), z);
 }
 
+// One warp's shared memory: NP-atom positions and the tables.
 template <int LPW, int NP>
-struct LjLaneWalker {
-  static constexpr int WPW = 32 / LPW;   // walkers per warp
-  static constexpr int APL = NP / LPW;   // atom slots per lane
-  float2* sp;                            // this warp's [3][APL][WPW][LPW] (hi, lo)
-  int slot;                              // this lane's walker within the warp
-  int glane;
-  unsigned gmask;
-  int n;
-  float wall_r2f;  // binary32 R^2 of the wall, set once per launch
-
-  __device__ float2& at(int c, int j) const {
-    return sp[((c * APL + j / LPW) * WPW + slot) * LPW + j % LPW];
-  }
-  __device__ void load(const float* p) {
-#pragma unroll
-    for (int k = 0; k < APL; ++k) {
-      const int j = glane + LPW * k;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) at(c, j) = make_float2(p[c * NP + j], p[(3 + c) * NP + j]);
-    }
-  }
-  __device__ void store(float* p, bool wr) const {
-    if (!wr) return;
-#pragma unroll
-    for (int k = 0; k < APL; ++k) {
-      const int j = glane + LPW * k;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float2 v = at(c, j);
-        p[c * NP + j] = v.x;
-        p[(3 + c) * NP + j] = v.y;
-      }
-    }
-  }
-  __device__ void put(int which, DS tx, DS ty, DS tz) {
-    if (glane == which % LPW) {
-      at(0, which) = make_float2(tx.h, tx.l);
-      at(1, which) = make_float2(ty.h, ty.l);
-      at(2, which) = make_float2(tz.h, tz.l);
-    }
-    if (LPW > 1) __syncwarp(gmask);  // the other lane reads the moved atom next move
-  }
-
-  // plan_move of lj.rs:365-374 and move_atom of lj.rs:86-105 for a given displacement:
-  // possible, and the energy change summed in binary32 over the walker's lanes.
-  __device__ bool plan(int which, float g0, float g1, float g2, float sh, float sl, double radius2,
-                       DS& tx, DS& ty, DS& tz, float& de_out) const {
-    const float2 a = at(0, which), b = at(1, which), c = at(2, which);
-    const DS fx{a.x, a.y}, fy{b.x, b.y}, fz{c.x, c.y};
-    tx = ds_add(fx, ds_scale(g0, sh, sl));
-    ty = ds_add(fy, ds_scale(g1, sh, sl));
-    tz = ds_add(fz, ds_scale(g2, sh, sl));
-    // wall: impossible iff |to|^2 > R^2 and |to|^2 > |from|^2 (lj.rs:87-90)
-    const float r2t = tx.h * tx.h + ty.h * ty.h + tz.h * tz.h;
-    const float r2f = fx.h * fx.h + fy.h * fy.h + fz.h * fz.h;
-    const float R2 = wall_r2f;
-    bool impossible;
-    if (r2t < R2 * (1.0f - 1e-5f)) {
-      impossible = false;
-    } else if (r2t > R2 * (1.0f + 1e-5f) && r2t > r2f * (1.0f + 1e-5f)) {
-      impossible = true;
-    } else {
-      const double x = ds_to_double(tx), y = ds_to_double(ty), z = ds_to_double(tz);
-      const double p = ds_to_double(fx), q = ds_to_double(fy), r = ds_to_double(fz);
-      const double nt = x * x + y * y + z * z, nf = p * p + q * q + r * r;
-      impossible = nt > radius2 && nt > nf;
-    }
-    if (impossible) return false;
-    float dn = 0.0f, dold = 0.0f;
-#pragma unroll
-    for (int k = 0; k < APL; ++k) {
-      const int j = glane + LPW * k;
-      if (j < n && j != which) {
-        const float2 xj = at(0, j), yj = at(1, j), zj = at(2, j);
-        // double-single differences: the high parts of nearby atoms subtract exactly
-        dn += lj_v32_fused((xj.x - tx.h) + (xj.y - tx.l), (yj.x - ty.h) + (yj.y - ty.l),
-                           (zj.x - tz.h) + (zj.y - tz.l));
-        dold += lj_v32_fused((xj.x - fx.h) + (xj.y - fx.l), (yj.x - fy.h) + (yj.y - fy.l),
-                             (zj.x - fz.h) + (zj.y - fz.l));
-      }
-    }
-    de_out = group_sum<LPW>(dn - dold, gmask);
-    return true;
-  }
-
-  // FP64 pair sum over the double-single positions (compute_energy, lj.rs:236-244).
-  __device__ double energy64() const {
-    double e = 0.0;
-#pragma unroll 1
-    for (int j = 0; j < n; ++j) {
-      const float2 a = at(0, j), b = at(1, j), c = at(2, j);
-      const double xj = (double)a.x + (double)a.y, yj = (double)b.x + (double)b.y,
-                   zj = (double)c.x + (double)c.y;
-#pragma unroll 4
-      for (int k = 0; k < APL; ++k) {
-        const int i = glane + LPW * k;
-        if (i < n && i > j) {
-          const float2 p = at(0, i), q = at(1, i), r = at(2, i);
-          const double dx = ((double)p.x + (double)p.y) - xj, dy = ((double)q.x + (double)q.y) - yj,
-                       dz = ((double)r.x + (double)r.y) - zj;
-          const double s = 1.0 / (dx * dx + dy * dy + dz * dz);
-          e += 4.0 * (powi6(s) - powi3(s));
-        }
-      }
-    }
-    return group_sum<LPW>(e, gmask);
+struct LjLaneShared {
+  static constexpr int PAIRS = NP / LPW / 2;  // slot pairs per lane
+  float2 pos[3][2][PAIRS][32];
+  float4 hi[32], lo[32];    // displacement of the batch's moves (hi.w: the atom, as int bits)
+  uint64_t u53[32];
+  RateTable rate;
+  double gamma[128];        // [walker][4 LPW]
+  __device__ float& at(int c, int part, int slot, int ln) {
+    float2& v = pos[c][part][slot >> 1][ln];
+    return slot & 1 ? v.y : v.x;
   }
 };
 
 template <int LPW, int NP, int FAM>
 __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
-  constexpr int WPW = 32 / LPW;
-  extern __shared__ float2 lane_smem[];
+  constexpr int WPW = 32 / LPW, APL = NP / LPW;
+  extern __shared__ __align__(16) unsigned char lane_smem[];
   const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;  // warp in block
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (warp * WPW >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
+  LjLaneShared<LPW, NP>& S = reinterpret_cast<LjLaneShared<LPW, NP>*>(lane_smem)[threadIdx.x >> 5];
   const int group = lane / LPW, glane = lane % LPW;
   int w = warp * WPW + group;
   const bool wr = w < m.n_walkers;
   if (!wr) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
 
-  Fh<LPW, FAM> fh;
+  Fh<LPW, FAM, BOOK_LEAN> fh;
   fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
-  LjLaneWalker<LPW, NP> lj;
-  lj.sp = lane_smem + (size_t)wib * 3 * NP * WPW;
-  lj.slot = group;
-  lj.glane = glane;
-  lj.gmask = gmask;
-  lj.n = fh.c.n;
-  lj.wall_r2f = __double2float_rn(s.radius2);
+  fh.gtab = S.gamma + group * 4 * LPW;
+  fh.lean_sync();
+  const int n = fh.c.n;
+  const float wall_r2f = __double2float_rn(s.radius2);
   float* pw = s.pos + (size_t)w * 6 * (size_t)NP;
-  lj.load(pw);
-  if (LPW > 1) __syncwarp();
+  for (int k = 0; k < APL; ++k)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int j = glane + LPW * k;
+      S.at(c, 0, k, lane) = pw[c * NP + j];
+      S.at(c, 1, k, lane) = pw[(3 + c) * NP + j];
+    }
+  // the slot pairs that hold atoms of any walker of the warp
+  int pairs = (n + 2 * LPW - 1) / (2 * LPW);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pairs = max(pairs, __shfl_xor_sync(0xffffffffu, pairs, o));
 
-  RecentScale rsb;
-  rsb.init();
   DS sc = ds_from_double(fh.c.tscale);
   Every resum;
   resum.init(fh.c.moves, m.resum_interval > 0 ? (uint64_t)m.resum_interval : 0);
-  // the draws of the next move are taken a move ahead, off the state's critical path
-  DrawCache<LPW, false> dc;
-  dc.init();
-  Draws nxt = dc.get(m.seed, (uint32_t)w, fh.c.moves + 1, (uint32_t)lj.n, gmask, glane);
-  for (uint64_t it = 0; it < m.n_moves; ++it) {
-    const uint64_t t = fh.c.moves + 1;
-    const Draws d = nxt;
-    if (it + 1 < m.n_moves) nxt = dc.get(m.seed, (uint32_t)w, t + 1, (uint32_t)lj.n, gmask, glane);
-    double rs, omrs;
-    rsb.get(t, lane, rs, omrs);
-    fh.begin_move(omrs);
-    DS tx, ty, tz;
-    float de = 0.0f;
-    const bool possible = lj.plan((int)d.which, d.g0, d.g1, d.g2, sc.h, sc.l, s.radius2, tx, ty, tz, de);
-    if (SADMC_RARE(m.trace && wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap)) {
-      TraceRec r;
-      r.e1 = fh.c.E;
-      r.e2 = possible ? fh.c.E + (double)de : __longlong_as_double(0x7ff8000000000000ll);
-      m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
+  Draws d{};  // of this lane's move in the batch of LPW
+  auto displace = [&]() {
+    const DS x = ds_scale(d.g0, sc.h, sc.l), y = ds_scale(d.g1, sc.h, sc.l), z = ds_scale(d.g2, sc.h, sc.l);
+    if (LPW > 1) __syncwarp(gmask);
+    S.hi[lane] = make_float4(x.h, y.h, z.h, __int_as_float((int)d.which));
+    S.lo[lane] = make_float4(x.l, y.l, z.l, 0.0f);
+    S.u53[lane] = d.u53;
+    if (LPW > 1) __syncwarp(gmask);
+  };
+  const F32x2 z{s.neg_zero2};
+  const uint32_t n_moves = (uint32_t)m.n_moves;
+  for (uint32_t it = 0; it < n_moves; ++it) {
+    const int kb = (int)(it % LPW);
+    if (kb == 0) {
+      d = draws_continuous(m.seed, (uint32_t)w, fh.c.moves + 1 + (uint64_t)glane, (uint32_t)n, 0u);
+      displace();
     }
-    const bool acc = fh.decide_de(possible, de, d.u53, rs);
-    if (acc) lj.put((int)d.which, tx, ty, tz);
-    fh.finish_move(acc);
-    if (SADMC_RARE(fh.tscale_changed)) { fh.tscale_changed = false; sc = ds_from_double(fh.c.tscale); }
+    const double2 rate = S.rate.get(it, fh.c.moves, lane);
+    fh.begin_move(rate.y);
+    // plan_move of lj.rs:365-374 and move_atom of lj.rs:86-105: the energy change summed in
+    // binary32 over the walker's lanes
+    const int e = group * LPW + kb;
+    const float4 gh = S.hi[e], gl = S.lo[e];
+    const uint64_t u53 = S.u53[e];
+    const int which = __float_as_int(gh.w);
+    const int wl = group * LPW + which % LPW, ws = which / LPW;
+    const DS fx{S.at(0, 0, ws, wl), S.at(0, 1, ws, wl)}, fy{S.at(1, 0, ws, wl), S.at(1, 1, ws, wl)},
+        fz{S.at(2, 0, ws, wl), S.at(2, 1, ws, wl)};
+    const DS tx = ds_add(fx, DS{gh.x, gl.x}), ty = ds_add(fy, DS{gh.y, gl.y}), tz = ds_add(fz, DS{gh.z, gl.z});
+    const bool possible = !lj_outside(tx, ty, tz, fx, fy, fz, wall_r2f, s.radius2);
+    const F32x2 tnh[3] = {f2_pack(-tx.h, -tx.h), f2_pack(-ty.h, -ty.h), f2_pack(-tz.h, -tz.h)},
+                tnl[3] = {f2_pack(-tx.l, -tx.l), f2_pack(-ty.l, -ty.l), f2_pack(-tz.l, -tz.l)},
+                fnh[3] = {f2_pack(-fx.h, -fx.h), f2_pack(-fy.h, -fy.h), f2_pack(-fz.h, -fz.h)},
+                fnl[3] = {f2_pack(-fx.l, -fx.l), f2_pack(-fy.l, -fy.l), f2_pack(-fz.l, -fz.l)};
+    float dn = 0.0f, dold = 0.0f;
+#pragma unroll 4
+    for (int p = 0; p < pairs; ++p) {
+      F32x2 ph[3], pl[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float2 h = S.pos[c][0][p][lane], l = S.pos[c][1][p][lane];
+        ph[c] = f2_pack(h.x, h.y);
+        pl[c] = f2_pack(l.x, l.y);
+      }
+      float n0, n1, o0, o1;
+      f2_unpack(lj_v32x2_fused(ph, pl, tnh, tnl, z), n0, n1);
+      f2_unpack(lj_v32x2_fused(ph, pl, fnh, fnl, z), o0, o1);
+      const int j0 = glane + LPW * 2 * p, j1 = j0 + LPW;
+      const bool on0 = j0 < n && j0 != which, on1 = j1 < n && j1 != which;
+      dn += on0 ? n0 : 0.0f;
+      dold += on0 ? o0 : 0.0f;
+      dn += on1 ? n1 : 0.0f;
+      dold += on1 ? o1 : 0.0f;
+    }
+    const float de = group_sum<LPW>(dn - dold, 0xffffffffu);
+    if (SADMC_RARE(m.trace != nullptr)) {
+      const uint64_t t = fh.c.moves;
+      if (wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
+        TraceRec r;
+        r.e1 = fh.c.E;
+        r.e2 = possible ? fh.c.E + (double)de : __longlong_as_double(0x7ff8000000000000ll);
+        m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
+      }
+    }
+    int r = fh.lean_decide(possible, de, u53);
+    if (SADMC_RARE(r == 2)) {
+      r = fh.decide_de(possible, de, u53, rate.x) ? 1 : 0;
+      fh.finish_move(r == 1);
+      fh.lean_sync();
+    } else {
+      const int old_cur = fh.cur;
+      if (r == 1) fh.lean_accept(de, rate.x);
+      fh.lean_finish(old_cur);
+    }
+    __syncwarp();
+    if (r == 1 && lane == wl) {
+      S.at(0, 0, ws, wl) = tx.h; S.at(0, 1, ws, wl) = tx.l;
+      S.at(1, 0, ws, wl) = ty.h; S.at(1, 1, ws, wl) = ty.l;
+      S.at(2, 0, ws, wl) = tz.h; S.at(2, 1, ws, wl) = tz.l;
+    }
+    __syncwarp();
+    if (SADMC_RARE(fh.tscale_changed)) {
+      fh.tscale_changed = false;
+      sc = ds_from_double(fh.c.tscale);
+      displace();  // the batch's remaining moves take the new scale
+    }
     if (SADMC_RARE(resum.tick())) {
-      const double e64 = lj.energy64();
+      // FP64 pair sum over the double-single positions (compute_energy, lj.rs:236-244)
+      double e64 = 0.0;
+#pragma unroll 1
+      for (int j = 0; j < n; ++j) {
+        const int jl = group * LPW + j % LPW, js = j / LPW;
+        const double xj = (double)S.at(0, 0, js, jl) + (double)S.at(0, 1, js, jl),
+                     yj = (double)S.at(1, 0, js, jl) + (double)S.at(1, 1, js, jl),
+                     zj = (double)S.at(2, 0, js, jl) + (double)S.at(2, 1, js, jl);
+#pragma unroll 4
+        for (int k = 0; k < APL; ++k) {
+          const int i = glane + LPW * k;
+          if (i < n && i > j) {
+            const double dx = ((double)S.at(0, 0, k, lane) + (double)S.at(0, 1, k, lane)) - xj,
+                         dy = ((double)S.at(1, 0, k, lane) + (double)S.at(1, 1, k, lane)) - yj,
+                         dz = ((double)S.at(2, 0, k, lane) + (double)S.at(2, 1, k, lane)) - zj;
+            const double q = 1.0 / (dx * dx + dy * dy + dz * dz);
+            e64 += 4.0 * (powi6(q) - powi3(q));
+          }
+        }
+      }
+      e64 = group_sum<LPW>(e64, gmask);
       const double dr = fabs(e64 - fh.c.E);
       if (dr > fh.c.drift) fh.c.drift = dr;
       if (dr > m.drift_tol) fh.c.status |= ST_DRIFT;
@@ -215,9 +216,18 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
         if (fh.grew_front) fh.reindex_after_growth();
         fh.move_cur(fh.gidx(e64));
       }
+      fh.lean_sync();
     }
   }
-  lj.store(pw, wr);
+  if (wr) {
+    for (int k = 0; k < APL; ++k)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int j = glane + LPW * k;
+        pw[c * NP + j] = S.at(c, 0, k, lane);
+        pw[(3 + c) * NP + j] = S.at(c, 1, k, lane);
+      }
+  }
   fh.store(m.cores, w);
 }
 
@@ -225,7 +235,7 @@ template <int LPW, int NP, int FAM>
 cudaError_t launch_lane(const MoveLaunch& m, const LjSys& s, cudaStream_t st) {
   constexpr int WPW = 32 / LPW;
   const int wpb = m.warps_per_block >= 1 && m.warps_per_block <= 4 ? m.warps_per_block : 1;
-  const size_t bytes = (size_t)wpb * 3 * NP * WPW * sizeof(float2);
+  const size_t bytes = (size_t)wpb * sizeof(LjLaneShared<LPW, NP>);
   // Larger than the default 48 KB for 64-atom walkers: the limit is raised once per device
   // (host threads may race to set it; setting it twice is harmless).
   static std::atomic<bool> attr[64] = {};
@@ -234,7 +244,7 @@ cudaError_t launch_lane(const MoveLaunch& m, const LjSys& s, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   if (device < 0 || device >= 64 || !attr[device].load(std::memory_order_acquire)) {
     e = cudaFuncSetAttribute(lj_lane_kernel<LPW, NP, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(4 * 3 * NP * WPW * sizeof(float2)));
+                             (int)(4 * sizeof(LjLaneShared<LPW, NP>)));
     if (e != cudaSuccess) return e;
     if (device >= 0 && device < 64) attr[device].store(true, std::memory_order_release);
   }
