@@ -81,12 +81,13 @@ struct sadmc_handle {
   int* d_cnt = nullptr;        // [W][cell_cap]
   int* d_atoms = nullptr;      // [W][cell_cap][bucket]
   int* d_build_status = nullptr;
+  uint64_t* d_words = nullptr; // [W][cell_cap], derived from the lists
   int cell_cap = 0, bucket = 16;
   double r_cut = 0.0;
   CellSys cell_sys() const {
     CellSys c{};
     c.pos = d_pos64; c.pos32 = d_pos32; c.np = np; c.box = d_box; c.ncell = d_ncell;
-    c.cell_of = d_cell_of; c.cell_count = d_cnt; c.cell_atoms = d_atoms; c.cell_cap = cell_cap;
+    c.cell_of = d_cell_of; c.cell_count = d_cnt; c.cell_atoms = d_atoms; c.words = d_words; c.cell_cap = cell_cap;
     c.bucket = bucket; c.r_cut = r_cut; c.kind = cfg.system; c.build_status = d_build_status;
     return c;
   }
@@ -465,6 +466,7 @@ int32_t sadmc_create(const sadmc_config* cfg, const sadmc_geometry* geom, sadmc_
            dalloc(&h->d_box, W * 3) == cudaSuccess && dalloc(&h->d_ncell, W * 3) == cudaSuccess &&
            dalloc(&h->d_cell_of, W * np) == cudaSuccess && dalloc(&h->d_cnt, W * cap) == cudaSuccess &&
            dalloc(&h->d_atoms, W * cap * h->bucket) == cudaSuccess &&
+           dalloc(&h->d_words, W * cap) == cudaSuccess &&
            dalloc(&h->d_build_status, W) == cudaSuccess;
       if (ok) {
         std::vector<double> box(W * 3);
@@ -497,6 +499,7 @@ int32_t sadmc_destroy(sadmc_handle* h) {
   cudaFree(h->d_trace_ds);
   cudaFree(h->d_pos64); cudaFree(h->d_pos32); cudaFree(h->d_box); cudaFree(h->d_ncell);
   cudaFree(h->d_cell_of); cudaFree(h->d_cnt); cudaFree(h->d_atoms); cudaFree(h->d_build_status);
+  cudaFree(h->d_words);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return SADMC_OK;
@@ -527,6 +530,7 @@ int32_t sadmc_upload_state(sadmc_handle* h, int32_t begin, int32_t count, const 
     int32_t r = h->prep_cores();
     if (r) return r;
     CUDA_TRY(launch_cell_build(h->d_cores, h->cell_sys(), h->W, h->stream));
+    CUDA_TRY(launch_cell_words(h->cell_sys(), h->W, h->stream));
     std::vector<int> st(h->W);
     CUDA_TRY(cudaMemcpyAsync(st.data(), h->d_build_status, sizeof(int) * h->W, cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -638,6 +642,7 @@ int32_t sadmc_initialize(sadmc_handle* h) {
       if (all) break;
       left -= m.n_moves;
     }
+    if (h->d_words) CUDA_TRY(launch_cell_words(h->cell_sys(), h->W, h->stream));  // it moved atoms
     if (c.system != SADMC_LJ) {
       // the descent accumulated energy changes; start from the FP64 energy of the result
       // (the LJ kernel re-sums itself)
@@ -1017,6 +1022,10 @@ int32_t sadmc_autotune(sadmc_handle* h, uint64_t moves, int32_t* best_lpw, doubl
       cudaError_t e = cudaMemcpyAsync(bufs[i].ptr, snap[i], bufs[i].bytes, cudaMemcpyDeviceToDevice, h->stream);
       if (e != cudaSuccess) return e;
     }
+    if (h->d_words) {
+      cudaError_t e = launch_cell_words(h->cell_sys(), h->W, h->stream);
+      if (e != cudaSuccess) return e;
+    }
     return cudaStreamSynchronize(h->stream);
   };
   cudaEvent_t e0, e1;
@@ -1133,6 +1142,7 @@ int32_t sadmc_resume(const char* path, sadmc_handle** out) {
         cudaMemcpy(b.ptr, host.data(), b.bytes, cudaMemcpyHostToDevice) != cudaSuccess) { ok = false; break; }
   }
   std::fclose(f);
+  if (ok && h->d_words && launch_cell_words(h->cell_sys(), W, h->stream) != cudaSuccess) ok = false;
   if (!ok) { sadmc_destroy(h); return fail(SADMC_ERR_INVALID, "truncated or mismatched checkpoint"); }
   h->uploaded = h->initialized = true;
   h->moves_done = moves_done;

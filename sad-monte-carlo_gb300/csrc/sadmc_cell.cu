@@ -53,6 +53,17 @@ __global__ void cell_build_kernel(const WalkerCore* cores, CellSys s, int n_walk
   }
 }
 
+// The buckets' words from their lists.
+__global__ void cell_words_kernel(CellSys s, size_t cells) {
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= cells) return;
+  const int c = (int)(k % s.cell_cap);
+  const int* nc = s.ncell + 3 * (k / s.cell_cap);
+  // a walker with fewer subcells than the largest leaves the rest of its row unused
+  const bool used = c < nc[0] * nc[1] * nc[2];
+  s.words[k] = used ? cell_word(s.cell_atoms + k * s.bucket, min(max(s.cell_count[k], 0), s.bucket)) : 0ull;
+}
+
 // compute_energy: WCA (wca.rs:222-230) and square well (optsquare.rs:176-186) in FP64
 // over the same candidate images.  One warp per walker.
 template <int KIND>
@@ -305,6 +316,12 @@ cudaError_t launch_cell_move(const MoveLaunch& m, const CellSys& s, int lpw, cud
 cudaError_t launch_cell_build(const WalkerCore* cores, const CellSys& s, int n_walkers,
                               cudaStream_t st) {
   dev::cell_build_kernel<<<(n_walkers + 127) / 128, 128, 0, st>>>(cores, s, n_walkers);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_cell_words(const CellSys& s, int n_walkers, cudaStream_t st) {
+  const size_t cells = (size_t)n_walkers * s.cell_cap;
+  dev::cell_words_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(s, cells);
   return cudaGetLastError();
 }
 

@@ -11,6 +11,14 @@
 // n_c >= 3 (geometries with fewer subcells are rejected: the reference double-counts
 // there, optcell.rs:343-346).
 //
+// What bounds the moves: a few warps per SM, each a chain of dependent instructions and loads.
+// Hence a move's query reads its neighbourhood in two loads (a subcell's bucket in one word,
+// then the atoms' positions), both positions share them when they share a subcell, the axes
+// run on three lanes at once, and the loops stay rolled: an unrolled scan ran twice as long
+// on the full batches (it outgrew the instruction cache).  Measured on one GB300: 2048 uneven
+// WCA walkers, 16 lanes, SAMC 9.9 -> 6.1 us per step; 1024 square-well walkers of 1024 atoms,
+// 32 lanes, WL 8.7 -> 5.4 us; the periodic FP64 re-sum of the WCA batch 3.7 -> 1.9 ms.
+//
 // Square well: overlap (r^2 < sigma^2) and contact (r^2 < lambda^2) decisions are those
 // of optsquare.rs:74-95 on the FP64 expression (p_j - off*L) - r, x*x + y*y + z*z.  They
 // are taken from binary32 copies when the binary32 r^2 lies outside a proven error
@@ -20,6 +28,9 @@
 // every resum_interval moves.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <atomic>
+#include <type_traits>
 
 #include "sadmc_common.cuh"
 #include "sadmc_fh.cuh"
@@ -340,9 +351,10 @@ struct CellOps {
   }
 };
 
-// FAM: the method the kernel is specialised for, or FAM_ANY (the method each walker holds).
-template <int LPW, int KIND, int FAM>
-__global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys s) {
+// The initial descent (energy.rs:840-851), over the bucket lists; the words are rebuilt after
+// it.
+template <int LPW, int KIND>
+__global__ void __launch_bounds__(128, 1) cell_descent_kernel(MoveLaunch m, CellSys s) {
   constexpr int WPW = 32 / LPW;
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -354,7 +366,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
   const unsigned gmask = group_mask<LPW>(group);
 
   __shared__ BucketScan sbs[128 / LPW];
-  Fh<LPW, FAM> fh;
+  Fh<LPW> fh;
   fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
   CellWalker cw;
   cw.np = s.np;
@@ -465,7 +477,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
     __syncwarp(gmask);
   };
 
-  if (m.descent) {
+  {
     // from_params descent (energy.rs:840-851): proposals of rms 0.05 on the descent stream,
     // confirmed when downhill; after every possible proposal the energy is tested against
     // max_allowed_energy (so at least one proposal is made).  WCA energy changes are the
@@ -504,38 +516,438 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
     fh.c.pad2 = steps;
     fh.c.pad1 = done ? 1 : 0;
     if (wr && glane == 0) m.cores[w] = fh.c;  // the host re-sums E in FP64 afterwards
-    return;
   }
+}
 
-  RecentScale rsb;
-  rsb.init();
-  DrawCache<LPW, false> dc;
-  dc.init();
+// A subcell's bucket in one word: its first four atoms, 12 bits each (at most 4096 atoms), and
+// its count in the top 16 bits.  A query reads the word in place of the count and of four list
+// entries; a fuller bucket's further atoms come from the list.
+__device__ __forceinline__ uint64_t cell_word(const int* list, int count) {
+  const int4 v = *reinterpret_cast<const int4*>(list);  // buckets are 16-byte aligned
+  const unsigned a = v.x & 0xfff, b = v.y & 0xfff, c = v.z & 0xfff, d = v.w & 0xfff;
+  return (uint64_t)a | ((uint64_t)b << 12) | ((uint64_t)c << 24) | ((uint64_t)d << 36) |
+         ((uint64_t)count << 48);
+}
+__device__ __forceinline__ int word_count(uint64_t w) { return (int)(w >> 48); }
+__device__ __forceinline__ int word_atom(uint64_t w, int s) { return (int)(w >> (12 * s)) & 0xfff; }
+
+// CellWalker::pair_sum64 over the words, for an f that is 0 from the cutoff on: a binary32
+// screen with a margin leaves out the candidates that would add nothing (five in six), which
+// spares their FP64 distances.  Same order, same bits.
+template <class F>
+__device__ double pair_sum64_screened(const CellWalker& cw, const uint64_t* words, int i, float reach, F f) {
+  const double qx = cw.p[i], qy = cw.p[cw.np + i], qz = cw.p[2 * cw.np + i];
+  const float4 qh = cw.p32[2 * i];
+  const int ci = cw.cell_of[i];
+  const int cx = ci / (cw.nc[1] * cw.nc[2]), cy = (ci / cw.nc[2]) % cw.nc[1], cz = ci % cw.nc[2];
+  double e = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < 27; ++k) {
+    int ux = cx + k / 9 - 1, uy = cy + (k / 3) % 3 - 1, uz = cz + k % 3 - 1;
+    const int ox = ux < 0 ? 1 : (ux >= cw.nc[0] ? -1 : 0), oy = uy < 0 ? 1 : (uy >= cw.nc[1] ? -1 : 0),
+              oz = uz < 0 ? 1 : (uz >= cw.nc[2] ? -1 : 0);
+    ux += ox * cw.nc[0]; uy += oy * cw.nc[1]; uz += oz * cw.nc[2];
+    const int c = cw.cell_index(ux, uy, uz);
+    const uint64_t word = words[c];
+    const int cnt = word_count(word);
+    const float sx = (float)ox * cw.L32[0] + qh.x, sy = (float)oy * cw.L32[1] + qh.y, sz = (float)oz * cw.L32[2] + qh.z;
+#pragma unroll 1
+    for (int q = 0; q < cnt; ++q) {
+      const int j = q < 4 ? word_atom(word, q) : cw.atoms[(size_t)c * cw.bucket + q];
+      const float4 pj = cw.p32[2 * j];
+      const float dx = pj.x - sx, dy = pj.y - sy, dz = pj.z - sz;
+      if (j == i || !(dx * dx + dy * dy + dz * dz < reach)) continue;
+      const double bx = (cw.p[j] - (double)ox * cw.L[0]) - qx;
+      const double by = (cw.p[cw.np + j] - (double)oy * cw.L[1]) - qy;
+      const double bz = (cw.p[2 * cw.np + j] - (double)oz * cw.L[2]) - qz;
+      e += f(bx * bx + by * by + bz * bz);
+    }
+  }
+  return e;
+}
+
+// One walker's proposal in shared memory, computed one axis per lane.
+struct CellNeighbour {  // one axis of a neighbour subcell
+  int index;            // its share of the subcell index
+  float off, shift;     // the image offset (-1, 0, 1) and the high part of off * L
+  int pad;
+};
+struct alignas(16) CellProposal {
+  double t[4];          // the new position
+  CellNeighbour nb[2][3][3 + 1];  // [new, old][axis][-1, 0, +1]
+  int cell[2][4];       // each axis's share of the new and the old position's subcell
+  float nh[4], oh[4];   // binary32 high parts of the two positions
+  float nl[4], ol[4];   // low parts (WCA)
+};
+// WCA: the pairs to evaluate of the two queries (0: the new position, 1: the old one).  v: first
+// what the screen found, a stretch of 16 per subcell for the lane that scans it, then the
+// energies; hit: atom | subcell << 12 | candidate index << 17, in the order of that index.  27
+// buckets of 16.
+struct CellPairs {
+  float v[2][432];
+  int hit[2][432];
+};
+struct CellNoPairs {};
+
+// A warp's shared memory.
+template <int LPW, int KIND>
+struct alignas(16) CellShared {
+  float4 g[32];         // the normals of a batch of LPW moves and the atom (as int bits)
+  uint64_t u53[32];
+  RateTable rate;
+  double gamma[128];
+  CellProposal prop[32 / LPW];
+  typename std::conditional<KIND == SYS_WCA, CellPairs, CellNoPairs>::type pairs[32 / LPW];
+};
+
+// The move kernel.  FAM: the method it is specialised for, or FAM_ANY (the method each walker
+// holds).  A lane takes whole subcells (k = lane, lane + LPW, ... of the 27), whose words and
+// atoms' positions it requests together, so that a query costs two loads in sequence; a
+// proposal that stays in its subcell, the common case, reads its neighbourhood once for both
+// positions.  The square well counts contacts in any order.  The WCA sum keeps the order in
+// which each lane took every LPW-th candidate: pairs that reach the cutoff are collected with
+// their index in that order, evaluated one per lane, and then summed in it.
+template <int LPW, int KIND, int FAM>
+__global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys s) {
+  constexpr int WPW = 32 / LPW, ROUNDS = (27 + LPW - 1) / LPW;
+  extern __shared__ __align__(16) unsigned char cell_smem[];
+  const int lane = threadIdx.x & 31;
+  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (warp * WPW >= m.n_walkers) return;
+  CellShared<LPW, KIND>& S = reinterpret_cast<CellShared<LPW, KIND>*>(cell_smem)[threadIdx.x >> 5];
+  const int group = lane / LPW, glane = lane % LPW;
+  int w = warp * WPW + group;
+  const bool wr = w < m.n_walkers;
+  if (!wr) w = m.n_walkers - 1;
+  const unsigned gmask = group_mask<LPW>(group);
+  CellProposal& P = S.prop[group];
+
+  Fh<LPW, FAM, BOOK_LEAN> fh;
+  fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
+  fh.gtab = S.gamma + group * 4 * LPW;
+  fh.lean_sync();
+  CellWalker cw;
+  cw.np = s.np;
+  cw.bucket = s.bucket;
+  cw.p = s.pos + (size_t)w * 3 * s.np;
+  cw.p32 = reinterpret_cast<float4*>(s.pos32) + (size_t)w * 2 * s.np;
+  cw.cell_of = s.cell_of + (size_t)w * s.np;
+  cw.cnt = s.cell_count + (size_t)w * s.cell_cap;
+  cw.atoms = s.cell_atoms + (size_t)w * s.cell_cap * s.bucket;
+  uint64_t* words = s.words + (size_t)w * s.cell_cap;
+  for (int a = 0; a < 3; ++a) {
+    cw.L[a] = s.box[3 * w + a];
+    cw.L32[a] = (float)cw.L[a];
+    cw.Ll32[a] = (float)(cw.L[a] - (double)cw.L32[a]);
+    cw.nc[a] = s.ncell[3 * w + a];
+  }
+  const int n = fh.c.n;
+  const double wsqr = s.r_cut * s.r_cut;
+  const float wsqr32 = (float)wsqr;
+  // the axis this lane computes (lanes 0-2 of a group)
+  const int ax = glane < 3 ? glane : 0;
+  const double axL = s.box[3 * w + ax];
+  const int axn = s.ncell[3 * w + ax];
+
+  // subcell k of query q's neighbourhood, and the axis indices (kx, ky, kz) of k in 0..2
+  auto split = [](int k, int& kx, int& ky, int& kz) {
+    kx = (k * 57) >> 9;  // k / 9 for k < 27
+    const int r = k - 9 * kx;
+    ky = (r * 11) >> 5;  // r / 3 for r < 9
+    kz = r - 3 * ky;
+  };
+  // this axis's stride in the subcell index
+  const int stride = ax == 0 ? cw.nc[1] * cw.nc[2] : (ax == 1 ? cw.nc[2] : 1);
+  const float axL32 = (float)axL;
+
   Every resum, datum;
   resum.init(fh.c.moves, KIND == SYS_WCA && m.resum_interval > 0 ? (uint64_t)m.resum_interval : 0);
   datum.init(fh.c.moves, KIND == SYS_WCA && m.B.ex_count ? (uint64_t)n * (uint64_t)n : 0);
-  for (uint64_t it = 0; it < m.n_moves; ++it) {
+  const uint32_t n_moves = (uint32_t)m.n_moves;
+  for (uint32_t it = 0; it < n_moves; ++it) {
+    const int kb = (int)(it % LPW);
     const uint64_t t = fh.c.moves + 1;
-    double rs, omrs;
-    rsb.get(t, lane, rs, omrs);
-    fh.begin_move(omrs);
-    const Draws d = dc.get(m.seed, (uint32_t)w, t, (uint32_t)n, gmask, glane);
-    const Prop p = plan((int)d.which, d.g0, d.g1, d.g2, fh.c.tscale);
-    if (m.trace && wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
+    const double2 rate = S.rate.get(it, fh.c.moves, lane);
+    if (kb == 0) {
+      const Draws d = draws_continuous(m.seed, (uint32_t)w, t + (uint64_t)glane, (uint32_t)n, 0u);
+      __syncwarp(gmask);
+      S.g[lane] = make_float4(d.g0, d.g1, d.g2, __int_as_float((int)d.which));
+      S.u53[lane] = d.u53;
+      __syncwarp(gmask);
+    }
+    fh.begin_move(rate.y);
+    const int e = group * LPW + kb;
+    const float4 g = S.g[e];
+    const uint64_t u53 = S.u53[e];
+    const int a = __float_as_int(g.w);
+    // plan_move: put_in_cell(from + g * scale) (optsquare.rs:273-284, wca.rs:342-353), one axis
+    // per lane
+    bool bad = false;
+    double tax;
+    {
+      const double f = cw.p[(size_t)ax * s.np + a];
+      const float ga = ax == 0 ? g.x : (ax == 1 ? g.y : g.z);
+      tax = wrap_axis(f + (double)ga * fh.c.tscale, axL, &bad);
+      if (glane < 3) {
+        P.t[ax] = tax;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          // inside the grid even where the wrap gave up (bad: the move is impossible)
+          const int cc = min(max(subcell_axis(q ? f : tax, axL, axn), 0), axn - 1);
+          P.cell[q][ax] = cc * stride;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const int u = cc + i - 1;
+            const bool lo = u < 0, hi = u >= axn;
+            CellNeighbour b;
+            b.index = (u + (lo ? axn : 0) - (hi ? axn : 0)) * stride;
+            b.off = lo ? 1.0f : (hi ? -1.0f : 0.0f);
+            b.shift = b.off * axL32;
+            b.pad = 0;
+            P.nb[q][ax][i] = b;
+          }
+        }
+        const float th = (float)tax, fhi = (float)f;
+        P.nh[ax] = th; P.oh[ax] = fhi;
+        if (KIND == SYS_WCA) { P.nl[ax] = (float)(tax - (double)th); P.ol[ax] = (float)(f - (double)fhi); }
+      }
+    }
+    const unsigned bads = __ballot_sync(0xffffffffu, bad);
+    bad = (bads & gmask) != 0;
+    const float4 nh = *reinterpret_cast<const float4*>(P.nh), oh = *reinterpret_cast<const float4*>(P.oh);
+    const int4 ni = *reinterpret_cast<const int4*>(P.cell[0]), oi = *reinterpret_cast<const int4*>(P.cell[1]);
+    const int new_c = ni.x + ni.y + ni.z, old_c = oi.x + oi.y + oi.z;
+    const bool stay = new_c == old_c;
+    bool possible = true;
+    float de = 0.0f;
+    // One pass over the 27 subcells serves both positions when they share a subcell; else the
+    // first pass is the new position's and the second the old one's.  The warp's walkers take
+    // their passes together.  (The loops are kept rolled: unrolled, the step's code outgrew the
+    // instruction cache.)
+    const int passes = __any_sync(0xffffffffu, !stay) ? 2 : 1;
+    // both positions' distances of an atom, shifted to its image, as a packed pair; screens
+    // only, whose margins cover any rounding
+    const F32x2 mx = f2_pack(-nh.x, -oh.x), my = f2_pack(-nh.y, -oh.y), mz = f2_pack(-nh.z, -oh.z);
+    auto dist2 = [&](float4 pj, float sx, float sy, float sz, float& dn, float& dp) {
+      const float x = pj.x - sx, y = pj.y - sy, z = pj.z - sz;
+      const F32x2 dx = f2_add(f2_pack(x, x), mx), dy = f2_add(f2_pack(y, y), my), dz = f2_add(f2_pack(z, z), mz);
+      f2_unpack(f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz, F32x2{0}))), dn, dp);
+    };
+    if (KIND == SYS_SW) {
+      // overlap (r^2 < 1) and contacts (r^2 < lambda^2) of optsquare.rs:74-95
+      int cn = 0, co = 0;
+      bool overlap = false;
+#pragma unroll 1
+      for (int p = 0; p < passes; ++p) {
+        const bool wn = p == 0, wo = stay == (p == 0);
+#pragma unroll 1
+        for (int k = glane * ROUNDS; k < min(glane * ROUNDS + ROUNDS, 27); ++k) {
+          int kx, ky, kz;
+          split(k, kx, ky, kz);
+          const CellNeighbour bx = P.nb[p][0][kx], by = P.nb[p][1][ky], bz = P.nb[p][2][kz];
+          const int c = bx.index + by.index + bz.index;
+          const uint64_t word = words[c];
+          const int cnt = wn || wo ? word_count(word) : 0;
+          auto take = [&](int j, float4 pj) {
+            float dn, dp;
+            dist2(pj, bx.shift, by.shift, bz.shift, dn, dp);
+            bool core = dn < 1.0f, hn = dn < wsqr32, ho = dp < wsqr32;
+            // within the binary32 margin of a threshold: the FP64 expression of
+            // optsquare.rs:78-86
+            if (SADMC_RARE(fminf(fminf(fabsf(dn - 1.0f), fabsf(dn - wsqr32)), fabsf(dp - wsqr32)) < 2e-4f)) {
+              const double ux = cw.p[j] - (double)bx.off * cw.L[0], uy = cw.p[cw.np + j] - (double)by.off * cw.L[1],
+                           uz = cw.p[2 * cw.np + j] - (double)bz.off * cw.L[2];
+              double ex = ux - P.t[0], ey = uy - P.t[1], ez = uz - P.t[2];
+              const double en = ex * ex + ey * ey + ez * ez;
+              ex = ux - cw.p[a]; ey = uy - cw.p[cw.np + a]; ez = uz - cw.p[2 * cw.np + a];
+              const double eo = ex * ex + ey * ey + ez * ez;
+              core = en < 1.0; hn = en < wsqr; ho = eo < wsqr;
+            }
+            const bool other = j != a;
+            overlap = overlap || (core && other && wn);
+            cn += hn && other && wn ? 1 : 0;
+            co += ho && other && wo ? 1 : 0;
+          };
+          float4 pj[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) pj[q] = cw.p32[q < cnt ? word_atom(word, q) : a];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) take(q < cnt ? word_atom(word, q) : a, pj[q]);
+#pragma unroll 1
+          for (int q = 4; q < cnt; ++q) {
+            const int j = cw.atoms[(size_t)c * cw.bucket + q];
+            take(j, cw.p32[j]);
+          }
+        }
+      }
+      // e = E - (contacts at the new position) + (contacts at the old position); the FP64
+      // sequence of unit steps of optsquare.rs:75-92 is exact on integers, and so is the
+      // binary32 difference of the two counts
+      __syncwarp();
+      de = (float)(LPW == 32 ? __reduce_add_sync(0xffffffffu, co - cn) : group_sum<LPW>(co - cn, 0xffffffffu));
+      possible = (__ballot_sync(0xffffffffu, overlap) & gmask) == 0;
+    } else {
+      CellPairs& T = *reinterpret_cast<CellPairs*>(&S.pairs[group]);
+      const float4 nl = *reinterpret_cast<const float4*>(P.nl), ol = *reinterpret_cast<const float4*>(P.ol);
+      // Screen the candidates on the high parts.  What comes within reach of the cutoff is noted
+      // with its ordinal in the lane; a prefix of the candidate and hit counts over the lanes,
+      // whose subcells are consecutive, then gives its index and its place in the list.
+      const float reach = wsqr32 + 1e-3f;
+      int total0 = 0, n0 = 0, n1 = 0;
+#pragma unroll 1
+      for (int p = 0; p < passes; ++p) {
+        const bool wn = p == 0, wo = stay == (p == 0);
+        const int k0 = glane * ROUNDS, k1 = wn || wo ? min(k0 + ROUNDS, 27) : 0;
+        int at = 0, h0 = 0, h1 = 0;
+#pragma unroll 1
+        for (int k = k0; k < k1; ++k) {
+          int kx, ky, kz;
+          split(k, kx, ky, kz);
+          const CellNeighbour bx = P.nb[p][0][kx], by = P.nb[p][1][ky], bz = P.nb[p][2][kz];
+          const int c = bx.index + by.index + bz.index;
+          const uint64_t word = words[c];
+          const int cnt = word_count(word);
+          auto take = [&](int q, int j, float4 pq) {
+            float dn, dp;
+            dist2(pq, bx.shift, by.shift, bz.shift, dn, dp);
+            const bool on = q < cnt && j != a;
+            const float code = __int_as_float(j | (k << 12) | ((at + q) << 17));
+            if (on && wn && dn < reach) T.v[0][k0 * 16 + h0++] = code;
+            if (on && wo && dp < reach) T.v[1][k0 * 16 + h1++] = code;
+          };
+          float4 pj[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) pj[q] = cw.p32[2 * (q < cnt ? word_atom(word, q) : a)];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) take(q, word_atom(word, q), pj[q]);
+#pragma unroll 1
+          for (int q = 4; q < cnt; ++q) {
+            const int j = cw.atoms[(size_t)c * cw.bucket + q];
+            take(q, j, cw.p32[2 * j]);
+          }
+          at += cnt;
+        }
+        __syncwarp();
+        // at most 432 of each
+        const int mine = at | (h0 << 10) | (h1 << 20);
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < LPW; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o, LPW);
+          if (glane >= o) incl += y;
+        }
+        const int all = __shfl_sync(0xffffffffu, incl, LPW - 1, LPW), before = incl - mine;
+        const int first = before & 1023;
+        if (h0 + h1 > 0) {
+          int* l0 = T.hit[0] + ((before >> 10) & 1023);
+          int* l1 = T.hit[1] + (before >> 20);
+#pragma unroll 1
+          for (int i = 0; i < h0; ++i) l0[i] = __float_as_int(T.v[0][k0 * 16 + i]) + (first << 17);
+#pragma unroll 1
+          for (int i = 0; i < h1; ++i) l1[i] = __float_as_int(T.v[1][k0 * 16 + i]) + (first << 17);
+        }
+        if (wn) { total0 = all & 1023; n0 = (all >> 10) & 1023; }
+        if (wo) n1 = all >> 20;
+      }
+      __syncwarp();
+      // pairs whose high-part r^2 may lie inside the cutoff (the high parts are within
+      // 2^-24 |L| of each coordinate), refined on the double-single positions
+#pragma unroll 1
+      for (int h = glane; h < n0 + n1; h += LPW) {
+        const bool oldq = h >= n0;
+        const int i = oldq ? h - n0 : h;
+        const int v = T.hit[oldq][i];
+        const int j = v & 0xfff;
+        int kx, ky, kz;
+        split((v >> 12) & 31, kx, ky, kz);
+        const int q = oldq && !stay ? 1 : 0;  // the pass that found it
+        const float fx = P.nb[q][0][kx].off, fy = P.nb[q][1][ky].off, fz = P.nb[q][2][kz].off;
+        const float4 pj = cw.p32[2 * j], pl = cw.p32[2 * j + 1];
+        const float rx = ds_image_diff(pj.x, pl.x, oldq ? oh.x : nh.x, oldq ? ol.x : nl.x, fx, cw.L32[0], cw.Ll32[0]);
+        const float ry = ds_image_diff(pj.y, pl.y, oldq ? oh.y : nh.y, oldq ? ol.y : nl.y, fy, cw.L32[1], cw.Ll32[1]);
+        const float rz = ds_image_diff(pj.z, pl.z, oldq ? oh.z : nh.z, oldq ? ol.z : nl.z, fz, cw.L32[2], cw.Ll32[2]);
+        T.v[oldq][i] = wca_v32(rx * rx + ry * ry + rz * rz, wsqr32);
+      }
+      __syncwarp();
+      // lane l takes candidates l, l + LPW, ... of the two queries' one list in turn; those that
+      // are not in the list add nothing
+      float e0 = 0.0f, e1 = 0.0f;
+#pragma unroll 1
+      for (int h = 0; h < n0; ++h)
+        if (((T.hit[0][h] >> 17) & (LPW - 1)) == glane) e0 += T.v[0][h];
+#pragma unroll 1
+      for (int h = 0; h < n1; ++h)
+        if ((((T.hit[1][h] >> 17) + total0) & (LPW - 1)) == glane) e1 += T.v[1][h];
+      __syncwarp();
+      de = group_sum<LPW>(e0 - e1, 0xffffffffu);
+    }
+    possible = possible && !bad && fabsf(de) <= 3.0e38f;
+    int new_count = 0;
+    if (!stay) {
+      new_count = word_count(words[new_c]);
+      if (SADMC_RARE(possible && new_count >= cw.bucket)) {
+        possible = false;
+        fh.c.status |= ST_CELL_OVERFLOW;
+      }
+    }
+    if (SADMC_RARE(m.trace && wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap)) {
       TraceRec r;
       r.e1 = fh.c.E;
-      r.e2 = p.possible ? fh.c.E + (double)p.de : __longlong_as_double(0x7ff8000000000000ll);
+      r.e2 = possible ? fh.c.E + (double)de : __longlong_as_double(0x7ff8000000000000ll);
       m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
     }
-    const bool acc = fh.decide_de(p.possible, p.de, d.u53, rs);
-    if (acc) apply(p);
-    fh.finish_move(acc);
-    if (datum.tick()) {
+    int r = fh.lean_decide(possible, de, u53);
+    if (SADMC_RARE(r == 2)) {
+      r = fh.decide_de(possible, de, u53, rate.x) ? 1 : 0;
+      fh.finish_move(r == 1);
+      fh.lean_sync();
+    } else {
+      const int old_cur = fh.cur;
+      if (r == 1) fh.lean_accept(de, rate.x);
+      fh.lean_finish(old_cur);
+    }
+    // ConfirmSystem::confirm -> Cell::move_atom (optcell.rs:162-175)
+    if (r == 1) {
+      if (SADMC_RARE(!stay)) {
+        int* lo = cw.atoms + (size_t)old_c * cw.bucket;
+        const int mo = min(word_count(words[old_c]), cw.bucket);
+        int pos = -1;
+        for (int k = glane; k < mo; k += LPW)
+          if (lo[k] == a) pos = k;
+#pragma unroll
+        for (int o = LPW / 2; o > 0; o >>= 1) {
+          const int x = __shfl_xor_sync(gmask, pos, o, LPW);
+          pos = x > pos ? x : pos;
+        }
+        __syncwarp(gmask);
+        if (wr && glane == 0 && pos >= 0) {
+          int* ln = cw.atoms + (size_t)new_c * cw.bucket;
+          lo[pos] = lo[mo - 1];
+          ln[new_count] = a;
+          cw.cnt[old_c] = mo - 1;
+          cw.cnt[new_c] = new_count + 1;
+          cw.cell_of[a] = new_c;
+          words[old_c] = cell_word(lo, mo - 1);
+          words[new_c] = cell_word(ln, new_count + 1);
+        }
+      }
+      if (wr && glane < 3) cw.p[(size_t)ax * s.np + a] = tax;
+      if (wr && glane == 0) {
+        if (KIND == SYS_WCA) {
+          cw.p32[2 * a] = make_float4(nh.x, nh.y, nh.z, 0.0f);
+          cw.p32[2 * a + 1] = make_float4(P.nl[0], P.nl[1], P.nl[2], 0.0f);
+        } else {
+          cw.p32[a] = make_float4(nh.x, nh.y, nh.z, 0.0f);
+        }
+      }
+    }
+    __syncwarp();
+    if (SADMC_RARE(datum.tick())) {
       // the "pressure" datum every N^2 moves into the current bin (wca.rs:202-218,
       // collected and binned as in energy.rs:944-946 and 374-386)
       double pv = 0.0;
       for (int i = glane; i < n; i += LPW)
-        pv += cw.pair_sum64(i, [&](double r2) { return wca_pressure64(r2, wsqr); });
+        pv += pair_sum64_screened(cw, words, i, wsqr32 + 1e-3f, [&](double r2) { return wca_pressure64(r2, wsqr); });
       pv = group_sum<LPW>(pv, gmask);
       if (wr && glane == 0) {
         const size_t k = (size_t)w * fh.nbins + fh.cur;
@@ -543,11 +955,11 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
         m.B.ex_total[k] += pv / (3.0 * (cw.L[0] * cw.L[1] * cw.L[2]));
       }
     }
-    if (resum.tick()) {
+    if (SADMC_RARE(resum.tick())) {
       // FP64 re-sum (wca.rs:222-230)
       double e = 0.0;
       for (int i = glane; i < n; i += LPW)
-        e += cw.pair_sum64(i, [&](double r2) { return wca_v64(r2, wsqr); });
+        e += pair_sum64_screened(cw, words, i, wsqr32 + 1e-3f, [&](double r2) { return wca_v64(r2, wsqr); });
       const double e64 = group_sum<LPW>(e, gmask) * 0.5;
       const double dr = fabs(e64 - fh.c.E);
       if (dr > fh.c.drift) fh.c.drift = dr;
@@ -559,6 +971,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
         if (fh.grew_front) fh.reindex_after_growth();
         fh.move_cur(fh.gidx(e64));
       }
+      fh.lean_sync();
     }
   }
   fh.store(m.cores, w);
@@ -566,14 +979,39 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
 
 }  // namespace dev
 
-// Launch cell_move_kernel<LPW, KIND, FAM> for the lanes per walker and the system.
-#define SADMC_CELL_CASE(L, K, F)                                                        \
-  if (lpw == L && s.kind == K) {                                                        \
-    const int warps = (m.n_walkers + (32 / L) - 1) / (32 / L);                          \
-    const int wpb = m.warps_per_block >= 1 && m.warps_per_block <= 4 ? m.warps_per_block : 4; \
-    dev::cell_move_kernel<L, K, F><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(m, s); \
-    return cudaGetLastError();                                                          \
+namespace dev {
+template <int LPW, int KIND, int FAM>
+cudaError_t launch_cell(const MoveLaunch& m, const CellSys& s, cudaStream_t st) {
+  const int warps = (m.n_walkers + (32 / LPW) - 1) / (32 / LPW);
+  int wpb = m.warps_per_block >= 1 && m.warps_per_block <= 4 ? m.warps_per_block : 4;
+  constexpr size_t per = sizeof(CellShared<LPW, KIND>);
+  constexpr int most = (int)(227 * 1024 / per) < 4 ? (int)(227 * 1024 / per) : 4;  // warps a block can hold
+  static_assert(most >= 1, "a warp's tables fit a block");
+  if (m.descent) {
+    cell_descent_kernel<LPW, KIND><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(m, s);
+    return cudaGetLastError();
   }
+  if (wpb > most) wpb = most;
+  // the shared-memory limit is raised once per device (host threads may race to set it;
+  // setting it twice is harmless)
+  static std::atomic<bool> attr[64] = {};
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  if (device < 0 || device >= 64 || !attr[device].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(cell_move_kernel<LPW, KIND, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(most * per));
+    if (e != cudaSuccess) return e;
+    if (device >= 0 && device < 64) attr[device].store(true, std::memory_order_release);
+  }
+  cell_move_kernel<LPW, KIND, FAM><<<(warps + wpb - 1) / wpb, 32 * wpb, wpb * per, st>>>(m, s);
+  return cudaGetLastError();
+}
+}  // namespace dev
+
+// Launch the move (or descent) kernel for the lanes per walker and the system.
+#define SADMC_CELL_CASE(L, K, F) \
+  if (lpw == L && s.kind == K) return dev::launch_cell<L, K, F>(m, s, st);
 #define SADMC_CELL_ALL_SHAPES(F)                                                        \
   SADMC_CELL_CASE(32, SYS_SW, F) SADMC_CELL_CASE(16, SYS_SW, F)                         \
   SADMC_CELL_CASE(8, SYS_SW, F) SADMC_CELL_CASE(4, SYS_SW, F)                           \

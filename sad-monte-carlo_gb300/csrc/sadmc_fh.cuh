@@ -234,6 +234,8 @@ struct Fh {
   float binB;           // distance from a bin edge, in bins, within which the estimate may err
   float tlof, invTf, lwlo, lwhi, belowB;  // too_lo, 1/min_T, ln w of the window's edge bins
   int lw_lo, lw_hi;     // the bins lwlo and lwhi were taken from
+  uint64_t k_wlh, p_wlh;  // WL: the stage histogram of the current and the proposed bin
+  bool wl_plain;        // WL: no production run, and the stage histogram spans the bins
   bool lean_off;        // every move takes the generic bookkeeping
   double* gtab;         // this walker's 4 LPW gammas in shared memory (LPW > 1)
 
@@ -725,6 +727,10 @@ struct Fh {
       lw_lo = win_lo; lw_hi = win_hi;
       cls = below(c.E, cur) ? -1 : (above(c.E, cur) ? 1 : 0);
     }
+    if (kind() == M_WL) {
+      wl_plain = !(c.has_min_gamma && c.gamma < c.min_gamma) && c.wl_hi - c.wl_lo == c.b_hi - c.b_lo;
+      if (wl_plain) k_wlh = wlh[c.wl_lo + (cur - c.b_lo)];
+    }
     lean_a1();
   }
   // ln w truncated to binary32 for 0 and [2^-126, 2^127): (double's bits >> 29) with the
@@ -773,6 +779,7 @@ struct Fh {
     // clamped into the allocated range, so that the loads stay inside it
     i2 = c.b_lo + min(max(qi, 0), c.b_hi - c.b_lo);
     p_lnw = lnw[i2]; p_hist = hist[i2]; p_stamp = stamp[i2];
+    if (kind() == M_WL && wl_plain) p_wlh = wlh[c.wl_lo + (i2 - c.b_lo)];
     float b2f = i2 == cur ? kf : lean_f32(p_lnw);
     float dd = ea;
     cls2 = 0;
@@ -807,6 +814,7 @@ struct Fh {
       flush_cur();
       cur = i2;
       k_lnw = p_lnw; k_hist = p_hist; k_stamp = p_stamp;
+      if (kind() == M_WL) k_wlh = p_wlh;
       kf = lean_f32(k_lnw);
     }
     cls = cls2;
@@ -837,9 +845,17 @@ struct Fh {
       if (SADMC_RARE(c.tL == c.moves)) sad_new_tF();
       if (cur == win_lo) lwlo = kf;
       if (cur == win_hi) lwhi = kf;
+    } else if (kind() == M_WL && wl_plain) {
+      k_lnw += c.gamma;
+      kf = lean_f32(k_lnw);
+      k_wlh += 1;
+      const uint64_t low = c.lowest_hist;
+      wl_count(c.wl_lo + (cur - c.b_lo), k_wlh);
+      if (SADMC_RARE(k_wlh == low + 1)) lean_sync();  // gamma and the histogram may have changed
     } else {
       update_weights(c.E);
       kf = lean_f32(k_lnw);
+      if (kind() == M_WL) lean_sync();  // a production run, or the histogram was regrouped
     }
     // energy.rs:950-965; truncation keeps the order of the weights
     const int li = cur - c.b_lo;
@@ -1009,7 +1025,6 @@ struct Fh {
   }
 
   __device__ void wl_update() {  // energy.rs:638-752
-    const bool inv_t = kind() == M_INV_T_WL;
     if (uni(c.has_min_gamma && c.gamma < c.min_gamma)) {  // production run
       int k = c.wl_lo + (cur - c.b_lo);
       if (k >= c.wl_lo && k <= c.wl_hi) { if (wr) wlh[k] = wlh[k] + 1; }
@@ -1052,10 +1067,18 @@ struct Fh {
       len_w = c.wl_hi - c.wl_lo + 1;
     }
     const int k = c.wl_lo + (cur - c.b_lo);
-    const uint64_t h = wlh[k] + 1;
+    wl_count(k, wlh[k] + 1);
+  }
+  // The stage histogram's new count h in plane bin k, and the flatness test
+  // (energy.rs:700-752).
+  __device__ void wl_count(int k, uint64_t h) {
+    const bool inv_t = kind() == M_INV_T_WL;
+    const int len_w = c.wl_hi - c.wl_lo + 1;
     if (wr) wlh[k] = h;
     if (h > c.wl_highest_hist) c.wl_highest_hist = h;
     c.total_hist += 1;
+    // only a bin that reaches the lowest count can change the outcome
+    if (!SADMC_RARE(uni(h == c.lowest_hist + 1))) return;
     const double max_energy = c.min_energy + (double)len_w * width;
     bool cond = h == c.lowest_hist + 1 && len_w > 1 &&
                 (!has_min_allowed || min_allowed >= c.min_energy) &&

@@ -81,6 +81,8 @@ struct CellSys {
   int* cell_of;       // [walker][np] subcell index of each atom
   int* cell_count;    // [walker][cell_cap]
   int* cell_atoms;    // [walker][cell_cap][bucket]
+  uint64_t* words;    // [walker][cell_cap] each bucket's count and first atoms (cell_word),
+                      // kept with the lists by the moves, else rebuilt from them
   int cell_cap;       // max subcells per walker
   int bucket;         // atom slots per subcell
   double r_cut;       // well width (square well) or 2^(1/6) (WCA)
@@ -89,6 +91,7 @@ struct CellSys {
 };
 cudaError_t launch_cell_build(const WalkerCore* cores, const CellSys& s, int n_walkers,
                               cudaStream_t st);
+cudaError_t launch_cell_words(const CellSys& s, int n_walkers, cudaStream_t st);
 cudaError_t launch_cell_move(const MoveLaunch& m, const CellSys& s, int lpw, cudaStream_t st);
 cudaError_t launch_cell_energy(const WalkerCore* cores, const CellSys& s, int n_walkers,
                                double* out, cudaStream_t st);
