@@ -322,6 +322,7 @@ struct sadmc_grand {
   double* d_pos64 = nullptr;
   float* d_pos32 = nullptr;
   int *d_cell_of = nullptr, *d_cnt = nullptr, *d_atoms = nullptr;
+  uint64_t* d_words = nullptr;
   int nc[3] = {0, 0, 0}, cell_cap = 0, bucket = 32;
   TraceRec* d_trace = nullptr;
   uint64_t trace_cap = 0, trace_t0 = 0, moves_done = 0;
@@ -343,7 +344,7 @@ struct sadmc_grand {
     m.drift_tol = cfg.drift_tol > 0 ? cfg.drift_tol : 1e-2;
     m.system = wca() ? 2 : 1;
     m.pos64 = d_pos64; m.pos32 = d_pos32; m.cell_of = d_cell_of; m.cell_count = d_cnt;
-    m.cell_atoms = d_atoms; m.cell_cap = cell_cap; m.bucket = bucket;
+    m.cell_atoms = d_atoms; m.words = d_words; m.cell_cap = cell_cap; m.bucket = bucket;
     for (int a = 0; a < 3; ++a) { m.box[a] = cfg.box[a]; m.nc[a] = nc[a]; }
     m.r_cut = std::pow(2.0, 1.0 / 6.0);
     return m;
@@ -1559,7 +1560,9 @@ int32_t sadmc_grand_create(const sadmc_grand_config* c, sadmc_grand** out) {
     if (e == cudaSuccess) e = cudaMalloc(&h->d_cell_of, sizeof(int) * W * h->np);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_cnt, sizeof(int) * W * h->cell_cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_atoms, sizeof(int) * W * h->cell_cap * h->bucket);
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_words, sizeof(uint64_t) * W * h->cell_cap);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->d_cnt, 0, sizeof(int) * W * h->cell_cap, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->d_words, 0, sizeof(uint64_t) * W * h->cell_cap, h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->d_pos64, 0, sizeof(double) * W * 3 * h->np, h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->d_pos32, 0, sizeof(float) * W * 8 * h->np, h->stream);
   }
@@ -1611,6 +1614,7 @@ int32_t sadmc_grand_destroy(sadmc_grand* h) {
   cudaFree(h->d_cell_of);
   cudaFree(h->d_cnt);
   cudaFree(h->d_atoms);
+  cudaFree(h->d_words);
   cudaFree(h->d_trace);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;

@@ -66,10 +66,12 @@ struct GrandLaunch {
   int* cell_of;
   int* cell_count;
   int* cell_atoms;
+  uint64_t* words;       // [walker][cells] each bucket's count and first atoms (cell_word)
   int cell_cap, bucket;
   double box[3];
   int nc[3];
   double r_cut;
+  unsigned long long neg_zero2 = 0x8000000080000000ull;  // two binary32 -0 (f2_mul)
 };
 
 cudaError_t launch_grand_move(const GrandLaunch& m, cudaStream_t st);

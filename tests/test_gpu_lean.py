@@ -3,6 +3,7 @@ the FP64 oracle, where its thresholds matter: bins too narrow for it, energy bou
 side or none, every method, ragged batches and launches that end inside a table batch."""
 import numpy as np
 import pytest
+from test_gpu_grand import SAME
 
 from helpers import METHOD_KW, assert_bins_equal, assert_scalars_equal, ising_spins, lj_configs
 
@@ -74,3 +75,39 @@ def test_ising_lean_path_bit_exact(gpu, oracle, method, energy_bin, bounds):
         assert_scalars_equal(b.scalars(w), ow.scalars(), label=f"walker {w}")
         np.testing.assert_array_equal(b.state(w), ow.state())
     assert not b.status().any()
+
+
+@pytest.mark.parametrize("box", [0.0, 4.5], ids=["lj", "wca"])
+@pytest.mark.parametrize("kw,lanes,max_N", [
+    (dict(energy_bin=0.02, min_allowed=-1.0, max_allowed=1.0), 8, 13),
+    (dict(energy_bin=0.5, min_allowed=-4.0, max_allowed=3.0, addremove_probability=0.9), 32, 13),
+    (dict(energy_bin=0.5, max_allowed=10.0, target_rate=0.5), 16, 40),     # the add/remove threshold moves
+    (dict(energy_bin=2.0, max_allowed=20.0, addremove_probability=0.5, method="wl"), 16, 40),
+    (dict(energy_bin=0.25, max_allowed=10.0), 32, 60)])
+def test_grand_lean_path(gpu, oracle, kw, lanes, max_N, box):
+    W, R, seed, runs = 5, 2.5, 9, (6000, 37, 3000)
+    kw = dict(dict(t0=500.0, translation_scale=0.1, addremove_probability=0.2, seed=seed), **kw)
+    kw["method"] = gpu.WL if kw.get("method") == "wl" else gpu.SAMC
+    geo = dict(box=(box,) * 3) if box else {}
+    e_lo, e_hi = (-1.0, 25.0) if box else (-200.0, 25.0)
+    b = gpu.GrandBatch(gpu.make_grand_config(W, max_N, **(geo or dict(radius=R)), e_lo=e_lo, e_hi=e_hi,
+                                             lanes_per_walker=lanes, **kw))
+    moves = sum(runs)
+    b.set_trace(moves)
+    for k in runs:
+        b.run(k)
+    for w in range(W):
+        gs = b.scalars(w)
+        assert gs["status"] == 0
+        e1, e2 = b.trace(w, moves)
+        ow = oracle.GrandWalker(oracle.make_grand_config(**(geo or dict(radius=R)), max_N=max_N, walker=w, **kw))
+        disc, mismatch = ow.run_override(e1, e2)
+        assert mismatch == 0 and disc < (5e-6 if box else 1e-5), (w, mismatch, disc, ow.worst())
+        gb, ob, os_ = b.bins(w), ow.bins(), ow.scalars()
+        for k in ("lnw", "hist", "visited", "round_trips"):
+            np.testing.assert_array_equal(gb[k], ob[k], err_msg=f"walker {w} {k}")
+        for k in SAME:
+            assert gs[k] == os_[k], (w, k, gs[k], os_[k])
+        for g, o in zip(b.translation_counts(w), ow.translation_counts()):
+            np.testing.assert_array_equal(g, o)
+        np.testing.assert_allclose(b.state(w), ow.state(), atol=1e-11)
