@@ -19,6 +19,7 @@
 #pragma once
 #include <cstdint>
 
+#include "sadmc_common.cuh"
 #include "sadmc_types.h"
 
 namespace sadmc {
@@ -221,6 +222,7 @@ struct Fh {
   int out_li, out_i1l;
   bool tsc_event;
   __device__ void invalidate_gamma() { gb_ok = 0; xg_ok = false; ++pgen; }
+  int wl_low;           // WL: visited bins whose stage count is at most lowest_hist (-1: to be counted)
   bool inverted;        // too_lo > too_hi (never true for SAD; kept exact)
   // LEAN: binary32 views of the state for lean_decide (lean_sync refreshes them after the
   // generic bookkeeping, lean_finish after an ordinary move)
@@ -364,6 +366,7 @@ struct Fh {
     tF_d = ns_d = 0.0;
     g_zero = true;
     lw_lo = lw_hi = -1;
+    wl_low = -1;
     xg = nullptr;
     xg_t0 = 0;
     xg_ok = false;
@@ -1037,6 +1040,7 @@ struct Fh {
       if (uni(len_w == 0 || (c.gamma != 1.0 && c.lowest_hist > 0))) {
         c.gamma = 1.0;
         c.lowest_hist = 0;
+        wl_low = -1;
         c.wl_highest_hist = 0;
         c.total_hist = 0;
         c.wl_lo = c.b_lo;
@@ -1063,6 +1067,7 @@ struct Fh {
           mn = h < mn ? h : mn;
         }
         c.lowest_hist = group_min(mn);
+        wl_low = -1;
       }
       len_w = c.wl_hi - c.wl_lo + 1;
     }
@@ -1077,25 +1082,30 @@ struct Fh {
     if (wr) wlh[k] = h;
     if (h > c.wl_highest_hist) c.wl_highest_hist = h;
     c.total_hist += 1;
-    // only a bin that reaches the lowest count can change the outcome
+    // The reference's minimum over the visited bins is lowest + 1 when none of them is at most
+    // lowest: their number is kept, so that the bins are gone over once per level and not at
+    // every bin that reaches it.  This bin joins them at its first visit and leaves them at
+    // lowest + 1.
+    if (wl_low >= 0) {
+      if (k_hist == 1) wl_low += h <= c.lowest_hist ? 1 : 0;
+      else wl_low -= h == c.lowest_hist + 1 ? 1 : 0;
+    }
     if (!SADMC_RARE(uni(h == c.lowest_hist + 1))) return;
     const double max_energy = c.min_energy + (double)len_w * width;
-    bool cond = h == c.lowest_hist + 1 && len_w > 1 &&
-                (!has_min_allowed || min_allowed >= c.min_energy) &&
+    bool cond = len_w > 1 && (!has_min_allowed || min_allowed >= c.min_energy) &&
                 (!has_max_allowed || max_allowed <= max_energy);
     if (uni(cond)) {
-      sync();
-      uint64_t mn = ~0ull;
-      for (int j = glane; j < len_w; j += LPW) {
-        if (ld_hist(c.b_lo + j) != 0) {
-          uint64_t v = wlh[c.wl_lo + j];
-          mn = v < mn ? v : mn;
-        }
+      if (uni(wl_low < 0)) {
+        sync();
+        int low = 0;
+        for (int j = glane; j < len_w; j += LPW)
+          if (ld_hist(c.b_lo + j) != 0 && wlh[c.wl_lo + j] <= c.lowest_hist) ++low;
+        wl_low = LPW > 1 ? group_sum<LPW>(low, gmask) : low;
       }
-      mn = group_min(mn);
-      cond = mn == c.lowest_hist + 1;
+      cond = wl_low == 0;
     }
     if (uni(cond)) {
+      wl_low = -1;
       c.lowest_hist = h;
       if ((inv_t && c.lowest_hist > 0) ||
           (double)c.lowest_hist >= 0.8 * (double)c.total_hist / c.wl_num_states) {
