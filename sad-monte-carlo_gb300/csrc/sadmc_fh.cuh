@@ -162,12 +162,15 @@ constexpr int FAM_ANY = -1;
 //  BOOK_LEAN   everything, with an ordinary move on the lean path (lean_decide, lean_finish).
 //              The energy sums are atomic additions that nothing waits for (one lane's
 //              additions to one address keep their order, so the sums round as sequential
-//              ones), and t_found is written where it is set instead of being cached.
-constexpr int BOOK_FULL = 0, BOOK_SPLIT = 1, BOOK_LEAN = 2;
-template <int LPW, int FAM = FAM_ANY, int MODE = BOOK_FULL>
+//              ones), and t_found is written where it is set instead of being cached;
+//  BOOK_LEAN_SHARED  the same for a walker whose planes are in shared memory, where an FP64
+//              atomic addition is a loop: the sums are cached with the current bin.
+constexpr int BOOK_FULL = 0, BOOK_SPLIT = 1, BOOK_LEAN = 2, BOOK_LEAN_SHARED = 3;
+// WHOLE: the system's energies are integers (see lean_sync).
+template <int LPW, int FAM = FAM_ANY, int MODE = BOOK_FULL, bool WHOLE = false>
 struct Fh {
-  static constexpr bool SPLIT = MODE == BOOK_SPLIT, LEAN = MODE == BOOK_LEAN;
-  static constexpr bool SUMS = MODE == BOOK_FULL;  // the energy sums are cached here
+  static constexpr bool SPLIT = MODE == BOOK_SPLIT, LEAN = MODE >= BOOK_LEAN;
+  static constexpr bool SUMS = MODE == BOOK_FULL || MODE == BOOK_LEAN_SHARED;  // the energy sums are cached here
   static_assert(!SPLIT || (LPW == 1 && FAM == M_SAD), "the split bookkeeping is SAD on one lane");
   WalkerCore c;
   // launch constants
@@ -694,20 +697,33 @@ struct Fh {
   // 4e-7, which also covers their own rounding.
   __device__ void lean_sync() {
     const float B = fmaxf(fmaxf(fabsf(cminf), fabsf(cmaxf)), fabsf(Ef)), u = 4.0e-7f;
-    const float tolB = 2.0f * B * u + 1e-30f;
-    in_lo = cminf + (tolB + fabsf(cminf) * u);
-    in_hi = cmaxf - (tolB + fabsf(cmaxf) * u);
+    // Integer energies that binary32 holds, with bin edges it holds at a power-of-two spacing:
+    // the estimates are exact, and so are the comparisons with a threshold it holds.  (An odd
+    // Ising lattice has its energies on the bin edges, where the margins would send every move to
+    // the general path: 64 walkers of 15 x 15, SAMC, 8192 moves, 25.7 ms with them, 14.6 exact.)
+    const bool exact = WHOLE && B < 4194304.0f && (double)cminf == c.cur_min && (double)cmaxf == cur_max &&
+                       (__float_as_uint(inv_wf) & 0x7fffffu) == 0u && (double)inv_wf * width == 1.0;
+    const float tolB = exact ? 0.0f : 2.0f * B * u + 1e-30f;
+    // how far an estimate must be from a threshold T to be on its side of it
+    auto margin = [&](float Tf, double T, float k) {
+      return exact && (double)Tf == T ? 0.0f : tolB + k * fabsf(Tf) * u + 1e-30f;
+    };
+    const float mc = margin(cminf, c.cur_min, 1.0f), mx = margin(cmaxf, cur_max, 1.0f);
+    in_lo = mc == 0.0f ? nextafterf(cminf, -INFINITY) : cminf + mc;  // e2 >= cur_min
+    in_hi = cmaxf - mx;                                             // e2 < cur_max
     out_hi = INFINITY; out_lo = -INFINITY;
     if (has_max_allowed) {
-      in_hi = fminf(in_hi, maxf - (tolB + fabsf(maxf) * u));
-      out_hi = maxf + (tolB + 3.0f * fabsf(maxf) * u);
+      const float m3 = margin(maxf, max_allowed, 3.0f);
+      in_hi = fminf(in_hi, m3 == 0.0f ? nextafterf(maxf, INFINITY) : maxf - m3);
+      out_hi = maxf + m3;
     }
     if (has_min_allowed) {
-      in_lo = fmaxf(in_lo, minf + (tolB + fabsf(minf) * u));
-      out_lo = minf - (tolB + 3.0f * fabsf(minf) * u);
+      const float m3 = margin(minf, min_allowed, 3.0f);
+      in_lo = fmaxf(in_lo, m3 == 0.0f ? nextafterf(minf, -INFINITY) : minf + m3);
+      out_lo = minf - m3;
     }
     tinyB = B * 1e-15f + 1e-37f;
-    binB = (tolB + fabsf(cminf) * u) * inv_wf + fabsf((cmaxf - cminf) * inv_wf) * u + 1e-6f;
+    binB = exact ? -1.0f : (tolB + fabsf(cminf) * u) * inv_wf + fabsf((cmaxf - cminf) * inv_wf) * u + 1e-6f;
     kf = lean_f32(k_lnw);
     maxSf = f32_trunc(c.max_S);
     ddB = fabsf(maxSf) * 6.0e-7f + 1e-30f;
@@ -718,9 +734,10 @@ struct Fh {
       lean_off = lean_off || inverted;
       const float thif = f32_trunc(c.too_hi);
       tlof = f32_trunc(c.too_lo);
-      const float ml = tolB + fabsf(tlof) * u, mh = tolB + fabsf(thif) * u;
-      win_in_lo = tlof + ml; win_out_lo = tlof - ml;
-      win_in_hi = thif - mh; win_out_hi = thif + mh;
+      const float ml = margin(tlof, c.too_lo, 1.0f), mh = margin(thif, c.too_hi, 1.0f);
+      win_out_lo = tlof - ml; win_out_hi = thif + mh;
+      win_in_lo = ml == 0.0f ? nextafterf(tlof, -INFINITY) : tlof + ml;
+      win_in_hi = mh == 0.0f ? nextafterf(thif, INFINITY) : thif - mh;
       invTf = (float)inv_minT;
       belowB = ml * invTf * 1.01f;
       if (cur == win_lo) lwlo = kf;
@@ -782,6 +799,7 @@ struct Fh {
     // clamped into the allocated range, so that the loads stay inside it
     i2 = c.b_lo + min(max(qi, 0), c.b_hi - c.b_lo);
     p_lnw = lnw[i2]; p_hist = hist[i2]; p_stamp = stamp[i2];
+    if (SUMS) { p_sE = sE[i2]; p_sE2 = sE2[i2]; }
     if (kind() == M_WL && wl_plain) p_wlh = wlh[c.wl_lo + (i2 - c.b_lo)];
     float b2f = i2 == cur ? kf : lean_f32(p_lnw);
     float dd = ea;
@@ -817,6 +835,7 @@ struct Fh {
       flush_cur();
       cur = i2;
       k_lnw = p_lnw; k_hist = p_hist; k_stamp = p_stamp;
+      if (SUMS) { k_sE = p_sE; k_sE2 = p_sE2; }
       if (kind() == M_WL) k_wlh = p_wlh;
       kf = lean_f32(k_lnw);
     }
@@ -872,8 +891,7 @@ struct Fh {
     } else if (SADMC_RARE(li == c.max_S_local)) {
       if (old_cur != cur) fill_visited(false);
     } else if (!visited_cur()) {
-      k_stamp = c.fill_gen;
-      if (wr) { stamp[cur] = c.fill_gen; rt[cur] = rt[cur] + 1; }
+      mark_visited();
     }
     lean_a1();
   }
@@ -907,11 +925,7 @@ struct Fh {
     const double E = c.E;
     if (SADMC_RARE(k_hist == 0)) set_found();
     k_hist += 1;
-    if (SUMS) {
-      k_sE += E;
-      k_sE2 += E2;  // E2 == E * E (set_E)
-    }
-    if (LEAN) add_sums();
+    if (!SPLIT) add_sums();
     if (SPLIT) tsc_event = false;
     update_weights(E);
     if (SPLIT) {
@@ -922,7 +936,13 @@ struct Fh {
     max_entropy(old_cur);
   }
   __device__ void add_sums() {  // energy.rs:941-942
-    if (wr && (LPW == 1 || glane == 0)) { atomicAdd(&sE[cur], c.E); atomicAdd(&sE2[cur], E2); }
+    if (SUMS) {
+      k_sE += c.E;
+      k_sE2 += E2;  // E2 == E * E (set_E)
+    } else if (wr && (LPW == 1 || glane == 0)) {
+      atomicAdd(&sE[cur], c.E);
+      atomicAdd(&sE2[cur], E2);
+    }
   }
   // energy.rs:950-965, old_cur the bin before the move
   __device__ void max_entropy(int old_cur) {
@@ -935,9 +955,12 @@ struct Fh {
       int i1 = grew_front ? gidx_exact(e1) : old_cur;
       if (i1 - c.b_lo != li) fill_visited(false);
     } else if (!visited_cur()) {
-      k_stamp = c.fill_gen;
-      if (wr) { stamp[cur] = c.fill_gen; rt[cur] = rt[cur] + 1; }
+      mark_visited();
     }
+  }
+  __device__ void mark_visited() {
+    k_stamp = c.fill_gen;
+    if (wr) { stamp[cur] = c.fill_gen; rt[cur] = rt[cur] + 1; }
   }
 
   // energy.rs:514-761

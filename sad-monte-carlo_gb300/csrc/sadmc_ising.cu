@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(128) ising_move_kernel(MoveLaunch m, IsingSys 
   const unsigned gmask = group_mask<LPW>(group);
   __shared__ RateTable rates[4];
   __shared__ double gammas[4][LPW > 1 ? 128 : 1];
-  Fh<LPW, FAM, BOOK_LEAN> fh;
+  Fh<LPW, FAM, BOOK_LEAN, true> fh;
   fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
   const int L = s.L;
   int8_t* S = s.spins + (size_t)w * (size_t)L * (size_t)L;

@@ -37,12 +37,14 @@ __host__ __device__ inline size_t ising_chain_bytes(int nbins, int L) {
   return (size_t)nbins * 64 + (((size_t)L * (size_t)L + 15) & ~(size_t)15) + sizeof(ChainTables);
 }
 
+// Bound by lane 0's instructions, about five cycles each.  An ordinary move takes the lean path:
+// one 15 x 15 walker, 8192 moves, Wang-Landau 12.3 -> 6.7 ms and SAMC 10.9 -> 7.0 ms.
 template <int FAM>
 __global__ void __launch_bounds__(32, 1) ising_chain_kernel(MoveLaunch m, IsingSys s) {
   extern __shared__ __align__(16) unsigned char stage[];
   const int lane = threadIdx.x;
   const int w = blockIdx.x;  // one walker per block of one warp
-  Fh<1, FAM> fh;
+  Fh<1, FAM, BOOK_LEAN_SHARED, true> fh;
   fh.load(m.cores, m.P, m.B, w, 1u << lane, 0, lane == 0);
   const int L = s.L;
   const int nb = m.P.nbins;
@@ -63,6 +65,7 @@ __global__ void __launch_bounds__(32, 1) ising_chain_kernel(MoveLaunch m, IsingS
   fh.hist = sq; fh.tf = sq + nb; fh.rt = sq + 2 * (size_t)nb; fh.wlh = sq + 3 * (size_t)nb;
   fh.stamp = sq + 4 * (size_t)nb;
   fh.xg = tb->gamma;
+  if (lane == 0) fh.lean_sync();
 
   for (uint64_t base = 0; base < m.n_moves; base += 32) {
     const int cnt = (int)(m.n_moves - base < 32 ? m.n_moves - base : 32);
@@ -108,9 +111,17 @@ __global__ void __launch_bounds__(32, 1) ising_chain_kernel(MoveLaunch m, IsingS
           r.e2 = fh.c.E + (double)de;
           m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
         }
-        const bool acc = fh.decide_de(true, de, tb->u53[k], tb->rs[k]);
-        if (acc) S[site] = (int8_t)(-sij);
-        fh.finish_move(acc);
+        int r = fh.lean_decide(true, de, tb->u53[k]);
+        if (SADMC_RARE(r == 2)) {
+          r = fh.decide_de(true, de, tb->u53[k], tb->rs[k]) ? 1 : 0;
+          fh.finish_move(r == 1);
+          fh.lean_sync();
+        } else {
+          const int old_cur = fh.cur;
+          if (r == 1) fh.lean_accept(de, tb->rs[k]);
+          fh.lean_finish(old_cur);
+        }
+        if (r == 1) S[site] = (int8_t)(-sij);
       }
     }
     __syncwarp();

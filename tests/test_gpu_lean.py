@@ -77,6 +77,33 @@ def test_ising_lean_path_bit_exact(gpu, oracle, method, energy_bin, bounds):
     assert not b.status().any()
 
 
+# An odd lattice has its energies on the bin edges, where the integer thresholds decide; one
+# walker runs its chain with the planes in shared memory.
+@pytest.mark.parametrize("method,L,W,energy_bin,bounds", [
+    ("sad", 15, 33, 1.0, None), ("samc", 9, 3, 4.0, (-101.0, 60.0)), ("wl", 15, 33, 8.0, None),
+    ("sad", 15, 3, 3.0, None), ("samc", 15, 1, 4.0, None), ("wl", 15, 1, 8.0, (-300.0, 200.0)),
+    ("inv_t_wl", 16, 1, 8.0, None), ("samc", 16, 1, 0.5, (-202.0, 98.0))])
+def test_ising_integer_thresholds(gpu, oracle, method, L, W, energy_bin, bounds):
+    N, seed = L * L, 17
+    kw = dict(METHOD_KW[method], energy_bin=energy_bin)
+    if bounds:
+        kw.update(min_allowed=bounds[0], max_allowed=bounds[1])
+    b = gpu.Batch(gpu.make_config(gpu.ISING, W, L, e_lo=-2.0 * N - 20, e_hi=2.0 * N + 20, seed=seed, **kw),
+                  [(L, 0.0, (0, 0, 0))] * W)
+    spins = [ising_spins(L, 700 + w) for w in range(W)]
+    b.upload(spins)
+    b.initialize()
+    for k in (7001, 33, 5000):
+        b.run(k)
+    for w in {0, W // 2, W - 1}:
+        ow = oracle.Walker(oracle.make_config(oracle.ISING, L, seed=seed, walker=w, **kw), spins[w])
+        ow.run(12034)
+        assert_bins_equal(b.bins(w), ow.bins(), label=f"walker {w}")
+        assert_scalars_equal(b.scalars(w), ow.scalars(), label=f"walker {w}")
+        np.testing.assert_array_equal(b.state(w), ow.state())
+    assert not b.status().any()
+
+
 @pytest.mark.parametrize("box", [0.0, 4.5], ids=["lj", "wca"])
 @pytest.mark.parametrize("kw,lanes,max_N", [
     (dict(energy_bin=0.02, min_allowed=-1.0, max_allowed=1.0), 8, 13),
