@@ -1424,18 +1424,11 @@ int32_t sadmc_surrogate_predict(sadmc_handle* h, const float* pos, int32_t confi
   unsigned int* flag = nullptr;
   CUDA_TRY(sg_timeout_flag(&flag));
   CUDA_TRY(cudaMemcpyAsync(h->sg_batch_pos, pos, sizeof(float) * 3 * rows, cudaMemcpyHostToDevice, h->stream));
-  CUDA_TRY(sg_descriptors(h->sg_batch_pos, n, (int)rows, sc.gq, nullptr, h->stream));
+  CUDA_TRY(sg_descriptors(h->sg_batch_pos, n, configs, sc.gq, h->stream));
   CUDA_TRY(sg_forward(sc.gq, (int)rows, h->sg_weights(), sc.e, flag, h->stream));
-  std::vector<float> e(rows);
-  CUDA_TRY(cudaMemcpyAsync(e.data(), sc.e, sizeof(float) * rows, cudaMemcpyDeviceToHost, h->stream));
-  int32_t r = sg_check_timeouts(h);
-  if (r) return r;
-  for (int c = 0; c < configs; ++c) {
-    double s = 0;
-    for (int i = 0; i < n; ++i) s += e[(size_t)c * n + i];
-    energies[c] = (float)s;
-  }
-  return SADMC_OK;
+  CUDA_TRY(sg_config_sums(sc.e, n, configs, h->sg_batch_e, h->stream));
+  CUDA_TRY(cudaMemcpyAsync(energies, h->sg_batch_e, sizeof(float) * configs, cudaMemcpyDeviceToHost, h->stream));
+  return sg_check_timeouts(h);
 }
 
 int32_t sadmc_draws(int32_t system, uint32_t n, uint64_t seed, uint32_t walker, uint64_t t0,

@@ -4,18 +4,34 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 
+#include "sadmc_common.cuh"
+
 namespace sadmc {
 namespace dev {
 
 __device__ __forceinline__ float rbf_centre(int k) { return 0.8f + (2.2f / 31.0f) * (float)k; }
 
-// SiLU z / (1 + e^-z) for the batched forward and the training kernels, with the hardware
-// reciprocal (__fdividef, a few ulp; 0 once the denominator passes 2^126, the SiLU's
-// limit for large negative z) in place of an IEEE division: the kernels evaluate a few
-// hundred SiLUs per thread in unrolled code, and the IEEE sequence's length made their
-// instruction fetch the limiter.  The error is far below the BF16 rounding of the
+// 2^x by the special-function unit; results below 2^-126 are zero.
+__device__ __forceinline__ float ex2_hw(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 2^x with subnormal results.
+__device__ __forceinline__ float ex2_sub(float x) {
+  float y;
+  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 1 / (1 + e^-z) on the special-function unit (0 once the denominator passes 2^126, the limit for
+// large negative z): the kernels evaluate a few hundred per thread, and an IEEE division's length
+// made their instruction fetch the limiter.  The error is far below the BF16 rounding of the
 // activations.
-__device__ __forceinline__ float silu32(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+__device__ __forceinline__ float sigmoid32(float z) {
+  return rcp_hw(1.0f + ex2_hw(-z * 1.4426950408889634f));  // e^-z = 2^(-z log2 e)
+}
+// SiLU z / (1 + e^-z) for the batched forward and the training kernels, and its derivative.
+__device__ __forceinline__ float silu32(float z) { return z * sigmoid32(z); }
 // SiLU as z/2 (1 + tanh(z/2)) on the hardware tanh (tanh.approx.f32, absolute error about
 // 2^-11): one special-function operation and an FMA in place of an exponential and an
 // IEEE division.  Used by the delayed-acceptance screen only, whose value decides no
@@ -26,8 +42,8 @@ __device__ __forceinline__ float silu_fast(float z) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
   return __fmaf_rn(h, t, h);
 }
-__device__ __forceinline__ float dsilu32(float z) {  // SiLU'(z), reciprocal as in silu32
-  const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+__device__ __forceinline__ float dsilu32(float z) {
+  const float s = sigmoid32(z);
   return s * (1.0f + z * (1.0f - s));
 }
 

@@ -94,8 +94,10 @@ constexpr size_t SG_STATIC_ROWS = 4096;
 // it; later calls on that device only read the cache.
 cudaError_t sg_static_scratch(void** out);
 
-cudaError_t sg_descriptors(const float* pos, int n, int rows, __nv_bfloat16* gq, float* gf,
-                           cudaStream_t st);
+// Descriptors of `configs` configurations of n atoms into gq [configs * n][32].
+cudaError_t sg_descriptors(const float* pos, int n, int configs, __nv_bfloat16* gq, cudaStream_t st);
+// out[c] = sum of configuration c's n per-row energies (FP64, row order).
+cudaError_t sg_config_sums(const float* e, int n, int configs, float* out, cudaStream_t st);
 // Batched forward on the tensor cores: per-row energies.  A tensor-core wait that runs
 // out writes NaN energies and, when timeout is not null, sets *timeout.
 cudaError_t sg_forward(const __nv_bfloat16* gq, int rows, const SgWeights& w, float* e,

@@ -67,3 +67,25 @@ def test_online_training_reduces_the_error(gpu, oracle):
     first = b.surrogate_train(1, batch=256, lr=2e-3, seed=1)
     last = b.surrogate_train(400, batch=256, lr=2e-3, seed=2)
     assert last < 0.2 * first, (first, last)
+
+
+@pytest.mark.parametrize("n,configs", [(2, 2600), (13, 10000), (38, 4000), (51, 2560), (53, 2600), (128, 2600)])
+def test_large_batches_match_small_ones(gpu, n, configs):
+    """A large batch takes a pair's descriptor terms once (while the sums of n atoms fit) and
+    several tiles per block; a small one each atom's by itself.  The arithmetic is the same."""
+    R = 1.2 * n ** (1 / 3)
+    b = gpu.Batch(gpu.make_config(gpu.LJ, 1, n, energy_bin=0.5, max_allowed=0.0, e_lo=-6.0 * n, e_hi=1.0, seed=2),
+                  [(n, R, (0, 0, 0))])
+    b.surrogate_init(seed=4, ring_capacity=16)
+    rng = np.random.default_rng(n)
+    b.surrogate_set_params(b.surrogate_params() + rng.normal(0, 0.05, b.SG_NPARAM).astype(np.float32))
+    pos = rng.normal(0, R / 2, (configs, n, 3)).astype(np.float32)
+    pos[5, 1] = pos[5, 0]      # coincident atoms
+    pos[6] *= 40               # beyond every radial function
+    got = b.surrogate_predict(pos)
+    small = np.concatenate([b.surrogate_predict(pos[k:k + 700]) for k in range(0, configs, 700)])
+    np.testing.assert_array_equal(got, small)
+    p = gpu.unpack_params(b.surrogate_params())
+    for k in (0, 5, 6, configs - 1):
+        want = M.forward(M.descriptors(pos[k].astype(np.float64)), p, emulate_bf16=True)[0].sum()
+        assert got[k] == pytest.approx(want, rel=2e-2, abs=2e-2 * np.abs(got).max())
