@@ -102,7 +102,7 @@ struct sadmc_handle {
   int wpb = 0;                                  // warps per block (0: the kernel's own default)
   // learned surrogate (LJ)
   float* sg_master = nullptr;                   // FP32 parameters
-  float* sg_grad = nullptr;
+  float* sg_grad = nullptr;                     // gradients, then the loss and the timeout flag taken
   float* sg_m = nullptr;
   float* sg_v = nullptr;
   __nv_bfloat16* sg_w1t = nullptr;              // bf16 copies for the tensor cores
@@ -116,16 +116,32 @@ struct sadmc_handle {
   float* sg_batch_pos = nullptr;                // gathered minibatch
   float* sg_batch_e = nullptr;
   int sg_batch_cap = 0;
-  double* sg_loss = nullptr;
-  unsigned int* sg_flag = nullptr;              // the timeout flag, read and cleared
+  double* sg_loss = nullptr;                    // inside sg_grad's allocation
+  unsigned int* sg_flag = nullptr;              // the timeout flag, read and cleared; likewise
+  unsigned int* sg_timeout = nullptr;           // the kernels' timeout flag
+  unsigned char* sg_host = nullptr;             // page-locked: results on their way to the caller
+  size_t sg_host_bytes = 0;
+  // gradients [SG_NPARAM], loss, flag
+  static constexpr size_t kSgLoss = (sizeof(float) * SG_NPARAM + 7) / 8 * 8, kSgFlag = kSgLoss + sizeof(double),
+                          kSgOut = kSgFlag + sizeof(unsigned int);
+  static constexpr size_t kSgEnergies = 16;     // sg_host of a prediction: the flag, then the energies
+  cudaError_t sg_reserve_host(size_t bytes) {
+    if (bytes <= sg_host_bytes) return cudaSuccess;
+    cudaFreeHost(sg_host);
+    sg_host = nullptr;
+    sg_host_bytes = 0;
+    cudaError_t e = cudaMallocHost(&sg_host, bytes);
+    if (e == cudaSuccess) sg_host_bytes = bytes;
+    return e;
+  }
   uint64_t* sg_stats = nullptr;                 // [W][2] delayed-acceptance counters
   SgWeights sg_weights() const { return SgWeights::from(sg_master, sg_w1t, sg_w2t, sg_wc); }
   SgAdam sg_adam(int step, float lr) const { return SgAdam{sg_master, sg_m, sg_v, step, lr}; }
   void free_surrogate() {
     cudaFree(sg_master); cudaFree(sg_grad); cudaFree(sg_m); cudaFree(sg_v); cudaFree(sg_w1t);
     cudaFree(sg_w2t); cudaFree(sg_wc); cudaFree(sg_ring_pos); cudaFree(sg_ring_e); cudaFree(sg_scratch);
-    cudaFree(sg_batch_pos); cudaFree(sg_batch_e); cudaFree(sg_loss); cudaFree(sg_flag); cudaFree(sg_stats);
-    sg_stats = nullptr;
+    cudaFree(sg_batch_pos); cudaFree(sg_batch_e); cudaFree(sg_stats); cudaFreeHost(sg_host);
+    sg_stats = nullptr; sg_host = nullptr; sg_host_bytes = 0;
     sg_master = sg_grad = sg_m = sg_v = sg_ring_pos = sg_ring_e = sg_batch_pos = sg_batch_e = nullptr;
     sg_w1t = sg_w2t = sg_wc = nullptr; sg_scratch = nullptr; sg_loss = nullptr; sg_flag = nullptr;
   }
@@ -1171,7 +1187,7 @@ int32_t sadmc_surrogate_init(sadmc_handle* h, uint64_t seed, int32_t ring_capaci
   h->free_surrogate();
   const int n = h->geom[0].n;
   cudaError_t e = cudaMalloc(&h->sg_master, sizeof(float) * SG_NPARAM);
-  if (e == cudaSuccess) e = cudaMalloc(&h->sg_grad, sizeof(float) * SG_NPARAM);
+  if (e == cudaSuccess) e = cudaMalloc(&h->sg_grad, sadmc_handle::kSgOut);
   if (e == cudaSuccess) e = cudaMalloc(&h->sg_m, sizeof(float) * SG_NPARAM);
   if (e == cudaSuccess) e = cudaMalloc(&h->sg_v, sizeof(float) * SG_NPARAM);
   if (e == cudaSuccess) e = cudaMalloc(&h->sg_w1t, sizeof(__nv_bfloat16) * SG_RBF * SG_H1);
@@ -1179,8 +1195,12 @@ int32_t sadmc_surrogate_init(sadmc_handle* h, uint64_t seed, int32_t ring_capaci
   if (e == cudaSuccess) e = cudaMalloc(&h->sg_wc, sizeof(__nv_bfloat16) * SG_WC_ELEMS);
   if (e == cudaSuccess) e = cudaMalloc(&h->sg_ring_pos, sizeof(float) * 3 * (size_t)n * ring_capacity);
   if (e == cudaSuccess) e = cudaMalloc(&h->sg_ring_e, sizeof(float) * ring_capacity);
-  if (e == cudaSuccess) e = cudaMalloc(&h->sg_loss, sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&h->sg_flag, sizeof(unsigned int));
+  if (e == cudaSuccess) e = h->sg_reserve_host(64 * 1024);
+  if (e == cudaSuccess) e = sg_timeout_flag(&h->sg_timeout);
+  if (e == cudaSuccess) {
+    h->sg_loss = reinterpret_cast<double*>(reinterpret_cast<char*>(h->sg_grad) + sadmc_handle::kSgLoss);
+    h->sg_flag = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(h->sg_grad) + sadmc_handle::kSgFlag);
+  }
   if (e != cudaSuccess) { h->free_surrogate(); return fail(SADMC_ERR_NOMEM, "surrogate allocation failed"); }
   // N(0, 1/fan_in) weights, zero biases (a splitmix/Box-Muller host generator)
   std::vector<float> p(SG_NPARAM, 0.0f);
@@ -1244,24 +1264,20 @@ cudaError_t sg_train_async(sadmc_handle* h, int steps, int batch, float lr, uint
   cudaError_t e = h->sg_reserve((size_t)batch * n, batch);
   if (e != cudaSuccess) return e;
   const SgScratch sc = SgScratch::carve(h->sg_scratch, (size_t)batch * n);
-  unsigned int* flag = nullptr;
-  e = sg_timeout_flag(&flag);
   for (int it = 0; it < steps && e == cudaSuccess; ++it) {
     e = sg_gather(h->sg_ring_pos, h->sg_ring_e, n, h->sg_count, seed, (uint64_t)it, batch, h->sg_batch_pos,
                   h->sg_batch_e, h->stream);
     h->sg_step += 1;
     if (e == cudaSuccess)
       e = sg_train_step(h->sg_batch_pos, h->sg_batch_e, batch, n, h->sg_weights(), h->sg_grad,
-                        h->sg_adam(h->sg_step, lr), sc, h->sg_loss, flag, h->stream);
+                        h->sg_adam(h->sg_step, lr), sc, h->sg_loss, h->sg_timeout, nullptr, h->stream);
   }
   return e;
 }
 
 // Synchronise the handle's stream and report (then clear) a tensor-core wait that ran out.
 int32_t sg_check_timeouts(sadmc_handle* h) {
-  unsigned int* flag = nullptr;
-  CUDA_TRY(sg_timeout_flag(&flag));
-  CUDA_TRY(sg_take_flag(flag, h->sg_flag, h->stream));
+  CUDA_TRY(sg_take_flag(h->sg_timeout, h->sg_flag, h->stream));
   unsigned int to = 0;
   CUDA_TRY(cudaMemcpyAsync(&to, h->sg_flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->stream));
   CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -1303,18 +1319,18 @@ int32_t sadmc_surrogate_loss_grads(sadmc_handle* h, const float* pos, const floa
   const int n = h->geom[0].n;
   CUDA_TRY(h->sg_reserve((size_t)configs * n, configs));
   const SgScratch sc = SgScratch::carve(h->sg_scratch, (size_t)configs * n);
-  unsigned int* flag = nullptr;
-  CUDA_TRY(sg_timeout_flag(&flag));
   CUDA_TRY(cudaMemcpyAsync(h->sg_batch_pos, pos, sizeof(float) * 3 * (size_t)configs * n, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(cudaMemcpyAsync(h->sg_batch_e, target, sizeof(float) * configs, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(sg_train_step(h->sg_batch_pos, h->sg_batch_e, configs, n, h->sg_weights(), h->sg_grad,
-                         h->sg_adam(0, 0.0f), sc, h->sg_loss, flag, h->stream));
-  double l = 0;
-  CUDA_TRY(cudaMemcpyAsync(&l, h->sg_loss, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  if (grads) CUDA_TRY(cudaMemcpyAsync(grads, h->sg_grad, sizeof(float) * SG_NPARAM, cudaMemcpyDeviceToHost, h->stream));
-  int32_t r = sg_check_timeouts(h);
-  if (r) return r;
-  if (loss) *loss = l;
+                         h->sg_adam(0, 0.0f), sc, h->sg_loss, h->sg_timeout, h->sg_flag, h->stream));
+  // gradients, loss and flag in one copy
+  CUDA_TRY(cudaMemcpyAsync(h->sg_host, h->sg_grad, sadmc_handle::kSgOut, cudaMemcpyDeviceToHost, h->stream));
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
+  unsigned int to = 0;
+  std::memcpy(&to, h->sg_host + sadmc_handle::kSgFlag, sizeof(to));
+  if (to) return fail(SADMC_ERR_CUDA, "a tensor-core wait of the surrogate ran out");
+  if (grads) std::memcpy(grads, h->sg_host, sizeof(float) * SG_NPARAM);
+  if (loss) std::memcpy(loss, h->sg_host + sadmc_handle::kSgLoss, sizeof(double));
   return SADMC_OK;
 }
 
@@ -1335,7 +1351,7 @@ int32_t sadmc_surrogate_loss_grads_noalloc(sadmc_handle* h, const float* pos, co
   // gradients only, no optimizer state touched; no timeout flag: a tensor-core wait that
   // ran out leaves NaN in the loss and the gradients, the only signal of this path
   CUDA_TRY(sg_train_step(pos, target, configs, h->geom[0].n, h->sg_weights(), grads, h->sg_adam(0, 0.0f),
-                         sc, loss, nullptr, st));
+                         sc, loss, nullptr, nullptr, st));
   return SADMC_OK;
 }
 
@@ -1420,15 +1436,20 @@ int32_t sadmc_surrogate_predict(sadmc_handle* h, const float* pos, int32_t confi
   const int n = h->geom[0].n;
   const size_t rows = (size_t)configs * n;
   CUDA_TRY(h->sg_reserve(rows, configs));
+  CUDA_TRY(h->sg_reserve_host(sadmc_handle::kSgEnergies + sizeof(float) * configs));
   const SgScratch sc = SgScratch::carve(h->sg_scratch, rows);
-  unsigned int* flag = nullptr;
-  CUDA_TRY(sg_timeout_flag(&flag));
   CUDA_TRY(cudaMemcpyAsync(h->sg_batch_pos, pos, sizeof(float) * 3 * rows, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(sg_descriptors(h->sg_batch_pos, n, configs, sc.gq, h->stream));
-  CUDA_TRY(sg_forward(sc.gq, (int)rows, h->sg_weights(), sc.e, flag, h->stream));
-  CUDA_TRY(sg_config_sums(sc.e, n, configs, h->sg_batch_e, h->stream));
-  CUDA_TRY(cudaMemcpyAsync(energies, h->sg_batch_e, sizeof(float) * configs, cudaMemcpyDeviceToHost, h->stream));
-  return sg_check_timeouts(h);
+  CUDA_TRY(sg_forward(sc.gq, (int)rows, h->sg_weights(), sc.e, h->sg_timeout, h->stream));
+  // the sums and the flag go straight to the page-locked buffer
+  float* out = reinterpret_cast<float*>(h->sg_host + sadmc_handle::kSgEnergies);
+  CUDA_TRY(sg_config_sums(sc.e, n, configs, out, h->sg_timeout, reinterpret_cast<unsigned int*>(h->sg_host), h->stream));
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
+  unsigned int to = 0;
+  std::memcpy(&to, h->sg_host, sizeof(to));
+  if (to) return fail(SADMC_ERR_CUDA, "a tensor-core wait of the surrogate ran out");
+  std::memcpy(energies, out, sizeof(float) * configs);
+  return SADMC_OK;
 }
 
 int32_t sadmc_draws(int32_t system, uint32_t n, uint64_t seed, uint32_t walker, uint64_t t0,

@@ -168,9 +168,11 @@ __global__ void __launch_bounds__(32 * DESC_WARPS) descriptor_pair_kernel(const 
 }
 
 // Energies of configurations: the FP64 sum of their rows in row order.  A block stages the rows of
-// SUM_CONFIGS configurations in shared memory; a thread each adds them.
+// SUM_CONFIGS configurations in shared memory; a thread each adds them.  The forward's timeout flag
+// is read and cleared into *flag_out.
 constexpr int SUM_CONFIGS = 64, SUM_THREADS = 256;
-__global__ void __launch_bounds__(SUM_THREADS) config_sum_kernel(const float* e, int n, int configs, float* out) {
+__global__ void __launch_bounds__(SUM_THREADS) config_sum_kernel(const float* e, int n, int configs, float* out,
+                                                                  unsigned int* timeout, unsigned int* flag_out) {
   extern __shared__ float se[];  // [SUM_CONFIGS][n | 1]
   const int c0 = blockIdx.x * SUM_CONFIGS, nc = min(SUM_CONFIGS, configs - c0), ld = n | 1;
   int c = threadIdx.x / n, i = threadIdx.x % n;
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(SUM_THREADS) config_sum_kernel(const float* e,
     if (i >= n) { i -= n; c += 1; }
   }
   __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *flag_out = atomicExch(timeout, 0u);
   if (threadIdx.x >= nc) return;
   double s = 0.0;
   for (int q = 0; q < n; ++q) s += (double)se[threadIdx.x * ld + q];
@@ -690,15 +693,16 @@ __device__ __forceinline__ void refresh_one(int p, float val, __nv_bfloat16* w1t
   }
 }
 
-// grad[p] = sum over tiles (fixed order) of part[t][p]; the last block sums the loss.  With
-// adam.step > 0, Adam (Kingma & Ba 2015) updates master[p] and the bf16 copies.
+// grad[p] = sum over tiles (fixed order) of part[t][p]; the last block sums the loss and, with
+// flag_out, reads and clears the timeout flag.  With adam.step > 0, Adam (Kingma & Ba 2015) updates master[p] and the bf16 copies.
 //
 // Bound by the latency of the loads: eight partial sums per parameter (tiles t = k mod 8),
 // combined in a fixed order, so that the result depends only on the number of tiles; warp k of a
 // block takes sum k of the block's 32 parameters (one thread for all eight, in 50 blocks, left
 // a chain of 21 rounds).  171 tiles: 18.2 -> 8.9 us.
 __global__ void __launch_bounds__(256) reduce_adam_kernel(const float* part, const double* lpart, int tiles,
-                                                          float* grad, double* loss, SgAdam adam,
+                                                          float* grad, double* loss, unsigned int* timeout,
+                                                          unsigned int* flag_out, SgAdam adam,
                                                           __nv_bfloat16* w1t, __nv_bfloat16* w2t,
                                                           __nv_bfloat16* wc) {
   __shared__ float a[8][32];
@@ -713,7 +717,10 @@ __global__ void __launch_bounds__(256) reduce_adam_kernel(const float* part, con
       if (threadIdx.x == 0)
         for (int t = 0; t < cnt; ++t) l += sl[t];
     }
-    if (threadIdx.x == 0) *loss = l;
+    if (threadIdx.x == 0) {
+      *loss = l;
+      if (flag_out) *flag_out = atomicExch(timeout, 0u);
+    }
     return;
   }
   const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -801,9 +808,10 @@ cudaError_t sg_descriptors(const float* pos, int n, int configs, __nv_bfloat16* 
   return cudaGetLastError();
 }
 
-cudaError_t sg_config_sums(const float* e, int n, int configs, float* out, cudaStream_t st) {
+cudaError_t sg_config_sums(const float* e, int n, int configs, float* out, unsigned int* timeout,
+                           unsigned int* flag_out, cudaStream_t st) {
   dev::config_sum_kernel<<<(configs + dev::SUM_CONFIGS - 1) / dev::SUM_CONFIGS, dev::SUM_THREADS,
-                           sizeof(float) * dev::SUM_CONFIGS * (n | 1), st>>>(e, n, configs, out);
+                           sizeof(float) * dev::SUM_CONFIGS * (n | 1), st>>>(e, n, configs, out, timeout, flag_out);
   return cudaGetLastError();
 }
 
@@ -871,7 +879,7 @@ cudaError_t sg_prepare_train(void) {
 
 cudaError_t sg_train_step(const float* pos, const float* target, int configs, int n,
                           const SgWeights& w, float* grad, const SgAdam& adam, SgScratch s,
-                          double* loss_dev, unsigned int* timeout, cudaStream_t st) {
+                          double* loss_dev, unsigned int* timeout, unsigned int* flag_out, cudaStream_t st) {
   if (n < 1 || n > SG_MAX_ATOMS || configs < 1) return cudaErrorInvalidValue;
   const int tiles = sg_tiles(configs, n);
   cudaError_t e = sg_prepare_train();
@@ -882,7 +890,7 @@ cudaError_t sg_train_step(const float* pos, const float* target, int configs, in
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
-    dev::reduce_adam_kernel<<<(SG_NPARAM + 31) / 32 + 1, 256, 0, st>>>(s.part, s.lpart, tiles, grad, loss_dev,
+    dev::reduce_adam_kernel<<<(SG_NPARAM + 31) / 32 + 1, 256, 0, st>>>(s.part, s.lpart, tiles, grad, loss_dev, timeout, flag_out,
                                                                     adam, w.w1t, w.w2t, w.wc);
     e = cudaGetLastError();
   }

@@ -96,8 +96,10 @@ cudaError_t sg_static_scratch(void** out);
 
 // Descriptors of `configs` configurations of n atoms into gq [configs * n][32].
 cudaError_t sg_descriptors(const float* pos, int n, int configs, __nv_bfloat16* gq, cudaStream_t st);
-// out[c] = sum of configuration c's n per-row energies (FP64, row order).
-cudaError_t sg_config_sums(const float* e, int n, int configs, float* out, cudaStream_t st);
+// out[c] = sum of configuration c's n per-row energies (FP64, row order); *timeout is read and
+// cleared into *flag_out.
+cudaError_t sg_config_sums(const float* e, int n, int configs, float* out, unsigned int* timeout,
+                           unsigned int* flag_out, cudaStream_t st);
 // Batched forward on the tensor cores: per-row energies.  A tensor-core wait that runs
 // out writes NaN energies and, when timeout is not null, sets *timeout.
 cudaError_t sg_forward(const __nv_bfloat16* gq, int rows, const SgWeights& w, float* e,
@@ -111,10 +113,11 @@ cudaError_t sg_take_flag(unsigned int* flag, unsigned int* out, cudaStream_t st)
 // per tile of whole configurations, then the gradient reduction over tiles into grad
 // and the loss (mean squared configuration-energy error) into *loss_dev; with
 // adam.step > 0 the same kernel takes the Adam step and refreshes the bf16 copies.
-// Deterministic: the tiles are summed in a fixed order.
+// Deterministic: the tiles are summed in a fixed order.  flag_out not null: *timeout is read and
+// cleared into it at the end.
 cudaError_t sg_train_step(const float* pos, const float* target, int configs, int n,
                           const SgWeights& w, float* grad, const SgAdam& adam, SgScratch s,
-                          double* loss_dev, unsigned int* timeout, cudaStream_t st);
+                          double* loss_dev, unsigned int* timeout, unsigned int* flag_out, cudaStream_t st);
 cudaError_t sg_refresh(const float* master, const SgWeights& w, cudaStream_t st);
 // Copy every walker's configuration (LJ double-single planes) and its energy (read from
 // the walker state on the device) into the training ring at ring_head.
