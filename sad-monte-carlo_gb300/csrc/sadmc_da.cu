@@ -46,13 +46,6 @@ inline size_t da_smem_bytes(int R) {
   return 4 * ((size_t)DA_W_WORDS + (size_t)DA_WPB * (size_t)da_walker_words(R));
 }
 
-// 2^x on the special-function unit (ex2.approx.ftz.f32, relative error about 2^-22)
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // Sum over the warp of v[l], left in lane l (a butterfly reduce-scatter: at each step a lane
 // keeps the half of its vector its partner sends it and adds the partner's copy of it).
 __device__ __forceinline__ float warp_reduce_scatter32(float (&v)[32], int lane) {
@@ -77,17 +70,25 @@ __device__ __forceinline__ void da_row_update(const float* sG, float* sGf, uint3
                                               float ro, float rn, float l2w, float (&acc)[KPL]) {
   const float4* gsrc = reinterpret_cast<const float4*>(sG + i * DA_GW + kb);
   float4* gdst = reinterpret_cast<float4*>(sGf + i * DA_GW + kb);
+  const F32x2 z = f2_pack(-0.0f, -0.0f), l2 = f2_pack(-l2w, -l2w), rn2 = f2_pack(rn, rn), ro2 = f2_pack(ro, ro);
 #pragma unroll
   for (int k4 = 0; k4 < KPL / 4; ++k4) {
     const float4 g = gsrc[k4];
     float o[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float cn = rbf_centre(kb + 4 * k4 + u);
-      const float pn = ex2_approx(-((rn - cn) * (rn - cn)) * l2w);
-      const float po = ex2_approx(-((ro - cn) * (ro - cn)) * l2w);
-      o[u] = (u == 0 ? g.x : u == 1 ? g.y : u == 2 ? g.z : g.w) + pn - po;
-      acc[4 * k4 + u] += pn;
+    for (int u = 0; u < 4; u += 2) {
+      const int k = kb + 4 * k4 + u;
+      const F32x2 c = f2_pack(-rbf_centre(k), -rbf_centre(k + 1));
+      const F32x2 dn = f2_add(rn2, c), dd = f2_add(ro2, c);
+      float n0, n1, o0, o1;
+      f2_unpack(f2_mul(f2_mul(dn, dn, z), l2, z), n0, n1);
+      f2_unpack(f2_mul(f2_mul(dd, dd, z), l2, z), o0, o1);
+      n0 = ex2_hw(n0); n1 = ex2_hw(n1);
+      const F32x2 pn = f2_pack(n0, n1), po = f2_pack(-ex2_hw(o0), -ex2_hw(o1));
+      const F32x2 gg = u == 0 ? f2_pack(g.x, g.y) : f2_pack(g.z, g.w);
+      f2_unpack(f2_add(f2_add(gg, pn), po), o[u], o[u + 1]);
+      acc[4 * k4 + u] += n0;
+      acc[4 * k4 + u + 1] += n1;
     }
     gdst[k4] = make_float4(o[0], o[1], o[2], o[3]);
     sGbw[i * DA_BW + kb / 2 + 2 * k4] = pack_bf16(o[0], o[1]);
@@ -128,12 +129,20 @@ __device__ __forceinline__ void da_slot1_packed(const LjWalker<32, APL>& lj, int
   }
 }
 
-template <int APL>
+// Bound by the number of warp instructions on a walker's chain, one warp per walker and fewer than
+// two warps per scheduler.  They were 3400 a move, 150 of them binary64, which an SM issues one
+// of in 19 clocks; now about 2600, a handful binary64: a move takes the lean path (lean_delayed),
+// RBF terms, SiLUs and pair energies are evaluated two at a time.  1024 walkers of 38 atoms:
+// 13.4 -> 7.4 us a move.  (A team of three warps per walker -- one deciding, two for the
+// descriptors, a tile each -- took 14.4: its longest chain is not much shorter, and the deciding
+// warp's state no longer fits its registers.)
+template <int APL, int FAM>
 __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys s, SgWeights wts, int R,
                                                              int refresh_interval, uint64_t* stats) {
   constexpr int GW = DA_GW;             // FP32 descriptor row stride (words)
   constexpr int BW = (SG_RBF + 2) / 2;  // bf16 descriptor row stride (words)
   extern __shared__ __align__(16) uint32_t da_smem[];
+  __shared__ double gammas[DA_WPB][128];  // Fh::gtab
   uint32_t* sW1 = da_smem;
   uint32_t* sW2 = sW1 + SG_H1 * MLP_S1;
   float* sb1 = reinterpret_cast<float*>(sW2 + SG_H2 * MLP_S2);
@@ -149,8 +158,10 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int w = blockIdx.x * DA_WPB + wib;
   if (w >= m.n_walkers) return;
-  Fh<32> fh;
+  Fh<32, FAM, BOOK_LEAN> fh;
   fh.load(m.cores, m.P, m.B, w, 0xffffffffu, lane, true);
+  fh.gtab = gammas[wib];
+  fh.lean_sync();
   LjWalker<32, APL> lj;
   lj.set_radius2(s.radius2);
   lj.glane = lane;
@@ -230,6 +241,7 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
   rsb.init();
   DrawCache<32, false> dc;
   dc.init();
+  uint64_t u2_all = 0, u2_t0 = ~0ull;  // the second-stage uniforms of 32 moves
   DS sc = ds_from_double(fh.c.tscale);
   uint64_t screened_out = 0, exact_evals = 0;
   Every resum, refresh_every;
@@ -241,10 +253,15 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
     rsb.get(t, lane, rs, omrs);
     fh.begin_move(omrs);
     const Draws d = dc.get(m.seed, (uint32_t)w, t, (uint32_t)n, 0xffffffffu, lane);
-    // second-stage uniform: its own Philox stream (counter word 2 = 4)
-    const Philox4 U = philox4x32_10(Philox4{(uint32_t)t, (uint32_t)(t >> 32), 4u, (uint32_t)(m.seed >> 32)},
-                                    (uint32_t)w, (uint32_t)m.seed);
-    const uint64_t u2 = u53_bits(U.x, U.y);
+    // second-stage uniform: its own Philox stream (counter word 2 = 4), a lane per move
+    if (SADMC_RARE(t - u2_t0 >= 32)) {
+      u2_t0 = t;
+      const uint64_t tl = t + (uint64_t)lane;
+      const Philox4 U = philox4x32_10(Philox4{(uint32_t)tl, (uint32_t)(tl >> 32), 4u, (uint32_t)(m.seed >> 32)},
+                                      (uint32_t)w, (uint32_t)m.seed);
+      u2_all = u53_bits(U.x, U.y);
+    }
+    const uint64_t u2 = __shfl_sync(0xffffffffu, u2_all, (int)(t - u2_t0));
     const int a = (int)d.which;
     DS fx, fy, fz;
     lj.fetch(a, fx, fy, fz);
@@ -286,55 +303,77 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
     }
     const float des = group_sum<32>(part, 0xffffffffu);
     const double e1 = fh.c.E;
-    const double e_til = e1 + (double)des;
-    if (m.trace && lane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
+    if (SADMC_RARE(m.trace && lane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap)) {
       // (E before, proposed E: NaN when screened out or impossible) and dS
       const size_t k = (size_t)w * m.trace_cap + (t - m.trace_t0 - 1);
       m.trace[k] = TraceRec{e1, __longlong_as_double(0x7ff8000000000000ll)};
       if (m.trace_ds) m.trace_ds[k] = des;
     }
-    const double lnw_cur = fh.lnw_current();
-    const double lnw_til = fh.lnw_at(e_til);
-    const bool uphill1 = dgt(lnw_til, lnw_cur);
-    const bool rej1 = fh.uni(uphill1 && metropolis_reject(lnw_cur - lnw_til, d.u53));
-    // a certain stage-1 acceptance consumed no randomness: stage 2 may use the move's own
-    // uniform (with a constant surrogate the chain is then the plain chain, bit for bit)
-    const uint64_t u_second = uphill1 ? u2 : d.u53;
-    bool acc = false;
-    if (rej1) {
-      ++screened_out;
-    } else {
-      // ---- stage 2: exact energy ----
-      ++exact_evals;
-      DS ux, uy, uz;
-      float de = 0.f;
-      const bool possible = lj.plan(a, d.g0, d.g1, d.g2, sc.h, sc.l, s.radius2, ux, uy, uz, de);
-      // Christen-Fox second stage for a state-dependent first stage: accept with
-      // min(1, [pi(y) a1(y,x)] / [pi(x) a1(x,y)]), pi = exp(-ln w(E)), where the first stage
-      // from x used E~ = E + dS and the reverse one from y would use e2 - dS:
-      //   ln a1(x,y) = min(0, ln w(E) - ln w(E~)),  ln a1(y,x) = min(0, ln w(e2) - ln w(e2 - dS)).
-      // decide_de accepts with min(1, exp(lnw_first - ln w(e2))), so
-      //   lnw_first = ln w(E) - ln a1(x,y) + ln a1(y,x).
-      // (A constant surrogate, dS = 0, gives ln w(E): the plain chain.)
-      double lnw_first = lnw_cur;
-      if (possible && fabsf(de) <= 3.0e38f) {
-        const double e2x = fh.c.E + (double)de;
-        const double back = fh.lnw_at(e2x) - fh.lnw_at(e2x - (double)des);
-        lnw_first = lnw_cur - (uphill1 ? lnw_cur - lnw_til : 0.0) + (back < 0.0 ? back : 0.0);
-      }
-      if (m.trace && lane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap)
-        m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)].e2 =
-            possible ? e1 + (double)de : __longlong_as_double(0x7ff8000000000000ll);
-      acc = fh.decide_de(possible, de, u_second, rs, true, lnw_first);
-      if (acc) {
-        lj.put(a, tx, ty, tz);
-        // every row < n of the proposed buffers was rewritten by this move: they become
-        // the current ones
-        float* t0 = sG; sG = sGf; sGf = t0;
-        float* t1 = sE; sE = sEn; sEn = t1;
-      }
+    // the exact energy of the second stage (also of a move that the first one screens out, whose
+    // share is too small to branch on)
+    float de = 0.f;
+    const bool possible = !lj_outside(tx, ty, tz, fx, fy, fz, lj.wall_r2f, s.radius2);
+    if (possible) {
+      const F32x2 tnh[3] = {f2_pack(-tx.h, -tx.h), f2_pack(-ty.h, -ty.h), f2_pack(-tz.h, -tz.h)},
+                  tnl[3] = {f2_pack(-tx.l, -tx.l), f2_pack(-ty.l, -ty.l), f2_pack(-tz.l, -tz.l)},
+                  fnh[3] = {f2_pack(-fx.h, -fx.h), f2_pack(-fy.h, -fy.h), f2_pack(-fz.h, -fz.h)},
+                  fnl[3] = {f2_pack(-fx.l, -fx.l), f2_pack(-fy.l, -fy.l), f2_pack(-fz.l, -fz.l)};
+      constexpr int k1 = APL - 1;
+      const F32x2 qh[3] = {f2_pack(lj.x[0].h, lj.x[k1].h), f2_pack(lj.y[0].h, lj.y[k1].h), f2_pack(lj.z[0].h, lj.z[k1].h)},
+                  ql[3] = {f2_pack(lj.x[0].l, lj.x[k1].l), f2_pack(lj.y[0].l, lj.y[k1].l), f2_pack(lj.z[0].l, lj.z[k1].l)};
+      float n0, n1, o0, o1;
+      f2_unpack(lj_v32x2(qh, ql, tnh, tnl, F32x2{s.neg_zero2}), n0, n1);
+      f2_unpack(lj_v32x2(qh, ql, fnh, fnl, F32x2{s.neg_zero2}), o0, o1);
+      de += lane < n && lane != a ? n0 - o0 : 0.0f;
+      if (APL > 1) de += lane + 32 < n && lane + 32 != a ? n1 - o1 : 0.0f;
+      de = group_sum<32>(de, 0xffffffffu);
     }
-    fh.finish_move(acc);
+    bool rej1, acc;
+    const int r = fh.lean_delayed(possible, de, des, d.u53, u2, rej1);
+    if (SADMC_RARE(r == 2)) {
+      const double lnw_cur = fh.lnw_current();
+      const double lnw_til = fh.lnw_at(e1 + (double)des);
+      const bool uphill1 = dgt(lnw_til, lnw_cur);
+      rej1 = fh.uni(uphill1 && metropolis_reject(lnw_cur - lnw_til, d.u53));
+      // a certain stage-1 acceptance consumed no randomness: stage 2 may use the move's own
+      // uniform (with a constant surrogate the chain is then the plain chain, bit for bit)
+      acc = false;
+      if (!rej1) {
+        // Christen-Fox second stage for a state-dependent first stage: accept with
+        // min(1, [pi(y) a1(y,x)] / [pi(x) a1(x,y)]), pi = exp(-ln w(E)), where the first stage
+        // from x used E~ = E + dS and the reverse one from y would use e2 - dS:
+        //   ln a1(x,y) = min(0, ln w(E) - ln w(E~)),  ln a1(y,x) = min(0, ln w(e2) - ln w(e2 - dS)).
+        // decide_de accepts with min(1, exp(lnw_first - ln w(e2))), so
+        //   lnw_first = ln w(E) - ln a1(x,y) + ln a1(y,x).
+        // (A constant surrogate, dS = 0, gives ln w(E): the plain chain.)
+        double lnw_first = lnw_cur;
+        if (possible && fabsf(de) <= 3.0e38f) {
+          const double e2x = fh.c.E + (double)de;
+          const double back = fh.lnw_at(e2x) - fh.lnw_at(e2x - (double)des);
+          lnw_first = lnw_cur - (uphill1 ? lnw_cur - lnw_til : 0.0) + (back < 0.0 ? back : 0.0);
+        }
+        acc = fh.decide_de(possible, de, uphill1 ? u2 : d.u53, rs, true, lnw_first);
+      }
+      fh.finish_move(acc);
+      fh.lean_sync();
+    } else {
+      acc = r == 1;
+      const int old_cur = fh.cur;
+      if (acc) fh.lean_accept(de, rs);
+      fh.lean_finish(old_cur);
+    }
+    if (rej1) ++screened_out;
+    else ++exact_evals;
+    if (SADMC_RARE(m.trace && lane == 0 && !rej1 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap))
+      m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)].e2 =
+          possible ? e1 + (double)de : __longlong_as_double(0x7ff8000000000000ll);
+    if (acc) {
+      lj.put(a, tx, ty, tz);
+      // every row < n of the proposed buffers was rewritten by this move: they become
+      // the current ones
+      float* t0 = sG; sG = sGf; sGf = t0;
+      float* t1 = sE; sE = sEn; sEn = t1;
+    }
     if (fh.tscale_changed) { fh.tscale_changed = false; sc = ds_from_double(fh.c.tscale); }
     if (resum.tick()) {
       const double e64 = lj.energy64();
@@ -348,6 +387,7 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
         if (fh.grew_front) fh.reindex_after_growth();
         fh.move_cur(fh.gidx(e64));
       }
+      fh.lean_sync();
     }
     if (refresh_every.tick()) refresh();
   }
@@ -360,6 +400,17 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
 }
 
 }  // namespace dev
+
+namespace {
+// SAD and SAMC have their own kernels: with the methods told apart at run time, a SAMC move of 40
+// atoms takes 8.7 us against 5.4 (9 walkers).
+using DaKernel = void (*)(MoveLaunch, LjSys, SgWeights, int, int, uint64_t*);
+DaKernel da_kernel(int shape, int method) {
+  if (method == M_SAD) return shape == 0 ? dev::lj_da_kernel<1, M_SAD> : dev::lj_da_kernel<2, M_SAD>;
+  if (method == M_SAMC) return shape == 0 ? dev::lj_da_kernel<1, M_SAMC> : dev::lj_da_kernel<2, M_SAMC>;
+  return shape == 0 ? dev::lj_da_kernel<1, dev::FAM_ANY> : dev::lj_da_kernel<2, dev::FAM_ANY>;
+}
+}  // namespace
 
 cudaError_t launch_lj_da(const MoveLaunch& m, const LjSys& s, const SgWeights& w, int max_atoms,
                          int refresh_interval, uint64_t* stats, cudaStream_t st) {
@@ -374,15 +425,16 @@ cudaError_t launch_lj_da(const MoveLaunch& m, const LjSys& s, const SgWeights& w
   const int shape = s.np == 32 ? 0 : 1;
   if (device < 0 || device >= 64 || !attr[device][shape].load(std::memory_order_acquire)) {
     const int lim = (int)dev::da_smem_bytes(s.np);
-    e = shape == 0 ? cudaFuncSetAttribute(dev::lj_da_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim)
-                   : cudaFuncSetAttribute(dev::lj_da_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    e = cudaSuccess;
+    for (int method : {(int)M_SAD, (int)M_SAMC, (int)M_WL})
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(da_kernel(shape, method), cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     if (e != cudaSuccess) return e;
     if (device >= 0 && device < 64) attr[device][shape].store(true, std::memory_order_release);
   }
   const size_t bytes = dev::da_smem_bytes(R);
   const int blocks = (m.n_walkers + dev::DA_WPB - 1) / dev::DA_WPB;
-  if (shape == 0) dev::lj_da_kernel<1><<<blocks, 32 * dev::DA_WPB, bytes, st>>>(m, s, w, R, refresh_interval, stats);
-  else dev::lj_da_kernel<2><<<blocks, 32 * dev::DA_WPB, bytes, st>>>(m, s, w, R, refresh_interval, stats);
+  da_kernel(shape, m.method)<<<blocks, 32 * dev::DA_WPB, bytes, st>>>(m, s, w, R, refresh_interval, stats);
   return cudaGetLastError();
 }
 

@@ -787,7 +787,13 @@ struct Fh {
   // is taken here from e2f = Ef + de against the moved thresholds; the Metropolis test from
   // the binary32 weights a, b with |(a - b) - (lnw1 - lnw2)| <= dd (see metropolis_reject2).
   // The proposed bin's fields are left in p_*.
+  // FIRST: the second stage of a delayed-acceptance move (see lean_delayed), whose test is on
+  // min(a - b, dmax).
   __device__ int lean_decide(bool possible, float de, uint64_t u53) {
+    return lean_test<false>(possible, de, u53, a1f, ea, 0.0f);
+  }
+  template <bool FIRST>
+  __device__ int lean_test(bool possible, float de, uint64_t u53, float a, float dd, float dmax) {
     const float e2f = Ef + de;
     const bool ordinary = e2f > in_lo && e2f < in_hi;
     const bool oob = (e2f > out_hi && de > tinyB) || (e2f < out_lo && de < -tinyB);
@@ -802,7 +808,6 @@ struct Fh {
     if (SUMS) { p_sE = sE[i2]; p_sE2 = sE2[i2]; }
     if (kind() == M_WL && wl_plain) p_wlh = wlh[c.wl_lo + (i2 - c.b_lo)];
     float b2f = i2 == cur ? kf : lean_f32(p_lnw);
-    float dd = ea;
     cls2 = 0;
     if (kind() == M_SAD && !(e2f > win_in_lo && e2f < win_in_hi)) {
       cls2 = e2f < win_out_lo ? -1 : (e2f > win_out_hi ? 1 : 0);
@@ -813,7 +818,8 @@ struct Fh {
       if (cls2 > 0) b2f = lwhi;
       if (cls2 < 0) { float eb; b2f = lean_below(e2f, eb); dd += eb; }
     }
-    const float df = a1f - b2f;
+    float df = a - b2f;
+    if (FIRST && dmax < df) df = dmax;
     const float e32 = __expf(df);
     const float mt = __fmaf_rn(fabsf(df), 6.0e-7f, __fmaf_rn(dd, 2.0f, 4.0e-6f));
     const float uf = (float)(uint32_t)(u53 >> 29) * (1.0f / 16777216.0f);  // u in [uf, uf + 2^-24)
@@ -823,6 +829,64 @@ struct Fh {
     if (SADMC_RARE(lean_off)) return 2;
     if (!possible || !(fabsf(de) <= 3.0e38f)) return 0;
     return decided ? (acc && !oob ? 1 : 0) : 2;
+  }
+  // lnw_at for E + d at its binary32 estimate ef, with the bound err of its error beyond a weight's
+  // own rounding; src tells equal sources apart (the plane's bin, or a negative number); false:
+  // undecided.
+  __device__ bool lean_lnw_at(float ef, float& wf, float& err, int& src) const {
+    err = 0.0f;
+    if (kind() == M_SAD && ef > win_out_hi) { wf = lwhi; src = -1; return true; }
+    if (kind() == M_SAD && ef < win_out_lo) { wf = lean_below(ef, err); src = -2; return wf == wf; }
+    const float q = (ef - cminf) * inv_wf;
+    const float qm = q + 12582912.0f, fr = q - (qm - 12582912.0f);
+    const int qi = __float_as_int(qm) - 0x4B400000 - (fr < 0.0f ? 1 : 0);
+    // how far ef must be from the allocated range's edges (see lean_sync)
+    const float m = (fabsf(cminf) + fabsf(cmaxf) + fabsf(Ef)) * 1.2e-6f + 1e-30f;
+    if (kind() != M_SAD && (ef < cminf - m || ef > cmaxf + m)) { wf = 0.0f; src = -3; return true; }
+    const bool sure = ef > cminf + m && ef < cmaxf - m && fabsf(fr) > binB &&
+                      (kind() != M_SAD || (ef > win_in_lo && ef < win_in_hi));
+    src = c.b_lo + min(max(qi, 0), c.b_hi - c.b_lo);
+    wf = src == cur ? kf : lean_f32(lnw[src]);
+    return sure && wf == wf;
+  }
+  // A delayed-acceptance move whose surrogate predicts the energy change des and whose exact one
+  // is de: 1 accepted, 0 rejected (screened: by the first stage), 2: for the general path.
+  //   first stage   ln w(E) - ln w(E + des) against u1, when that is negative (uphill);
+  //   second stage  accepts with min(1, exp(f - ln w(e2))), e2 = E + de,
+  //                 f = A + min(0, ln w(e2) - ln w(e2 - des)), A = ln w(E + des) if uphill,
+  //                 else ln w(E): the exponent is min(A - ln w(e2), A - ln w(e2 - des)).
+  // u2 is the second stage's uniform after an uphill first stage; otherwise it is u1.
+  __device__ int lean_delayed(bool possible, float de, float des, uint64_t u1, uint64_t u2, bool& screened) {
+    screened = false;
+    if (SADMC_RARE(lean_off)) return 2;
+    float tw, te, bw = 0.0f, be = 0.0f;
+    int ts, bs;
+    if (SADMC_RARE(!lean_lnw_at(Ef + des, tw, te, ts))) return 2;
+    const bool same = cls == 0 ? ts == cur : (cls > 0 ? ts == -1 : false);
+    const float df = a1f - tw, dd = ea + te;
+    bool uphill = false;
+    if (!same) {
+      const float tol = __fmaf_rn(fabsf(df), 6.0e-7f, dd);
+      if (SADMC_RARE(!(fabsf(df) > tol))) return 2;
+      uphill = df < 0.0f;
+      if (uphill) {
+        const float e32 = __expf(df);
+        const float mt = __fmaf_rn(fabsf(df), 6.0e-7f, __fmaf_rn(dd, 2.0f, 4.0e-6f));
+        const float uf = (float)(uint32_t)(u1 >> 29) * (1.0f / 16777216.0f);
+        if (uf > __fmaf_rn(e32, mt, e32)) { screened = true; return 0; }
+        if (SADMC_RARE(!(uf + (1.0f / 16777216.0f) < __fmaf_rn(-e32, mt, e32)) || !(dd < 0.25f))) return 2;
+      }
+    }
+    if (!possible || !(fabsf(de) <= 3.0e38f)) return 0;
+    const bool sure = lean_lnw_at((Ef + de) - des, bw, be, bs);
+    const float A = uphill ? tw : a1f;
+    const int r = lean_test<true>(true, de, uphill ? u2 : u1, A, dd + be, A - bw);
+    // an energy out of bounds is rejected whatever the weights are
+    return SADMC_RARE(!sure) ? (r == 0 && lean_out(de) ? 0 : 2) : r;
+  }
+  __device__ bool lean_out(float de) const {
+    const float e2f = Ef + de;
+    return (e2f > out_hi && de > tinyB) || (e2f < out_lo && de < -tinyB);
   }
   // An accepted lean move: the counters and the state of the proposed bin.
   __device__ void lean_accept(float de, double rs) {

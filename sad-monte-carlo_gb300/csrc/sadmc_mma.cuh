@@ -33,14 +33,22 @@ __device__ __forceinline__ float sigmoid32(float z) {
 // SiLU z / (1 + e^-z) for the batched forward and the training kernels, and its derivative.
 __device__ __forceinline__ float silu32(float z) { return z * sigmoid32(z); }
 // SiLU as z/2 (1 + tanh(z/2)) on the hardware tanh (tanh.approx.f32, absolute error about
-// 2^-11): one special-function operation and an FMA in place of an exponential and an
-// IEEE division.  Used by the delayed-acceptance screen only, whose value decides no
-// move by itself (the exact energy makes every final decision).
-__device__ __forceinline__ float silu_fast(float z) {
-  const float h = 0.5f * z;
+// 2^-11), of c + b for two units at once: one special-function operation and an FMA in place of an
+// exponential and an IEEE division.  Used by the delayed-acceptance screen only, whose value
+// decides no move by itself (the exact energy makes every final decision).
+__device__ __forceinline__ float tanh_hw(float x) {
   float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
-  return __fmaf_rn(h, t, h);
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(x));
+  return t;
+}
+__device__ __forceinline__ float2 silu_fast2(float c0, float c1, float2 b) {
+  const F32x2 zero = f2_pack(-0.0f, -0.0f);
+  const F32x2 h = f2_mul(f2_pack(0.5f, 0.5f), f2_add(f2_pack(c0, c1), f2_pack(b.x, b.y)), zero);
+  float x, y;
+  f2_unpack(h, x, y);
+  float2 r;
+  f2_unpack(f2_fma(h, f2_pack(tanh_hw(x), tanh_hw(y)), h), r.x, r.y);
+  return r;
 }
 __device__ __forceinline__ float dsilu32(float z) {
   const float s = sigmoid32(z);
@@ -80,7 +88,7 @@ __host__ __device__ constexpr int mlp_wword(int n, int w, int stride) {
 
 // Surrogate energies of 16 rows (one warp): A fragments of G from a row-major bf16 tile
 // in shared memory (32 bf16 = 16 words per row), weights in the mlp_wword layout and biases
-// as float pairs in shared memory, SiLU in its tanh form (silu_fast).  Rows g and g+8 of
+// as float pairs in shared memory, SiLU in its tanh form (silu_fast2).  Rows g and g+8 of
 // the tile end in ea / eb (in the quad's lane t == 0 and the others alike).
 template <int RW>  // 32-bit words between consecutive rows of the tile
 __device__ __forceinline__ void mlp16(const uint32_t* gtile, const uint2* sW1, const uint2* sW2,
@@ -95,7 +103,7 @@ __device__ __forceinline__ void mlp16(const uint32_t* gtile, const uint2* sW1, c
     aG[kt][2] = gtile[g * RW + 8 * kt + 4 + t];
     aG[kt][3] = gtile[(g + 8) * RW + 8 * kt + 4 + t];
   }
-  float h1[8][4];
+  uint32_t h1[8][2];  // units 8 j + 2 t, + 1 of rows g and g + 8, as layer 2 takes them
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     float c[4] = {0.f, 0.f, 0.f, 0.f};
@@ -106,29 +114,29 @@ __device__ __forceinline__ void mlp16(const uint32_t* gtile, const uint2* sW1, c
       mma16816(c, aG[kt], b.x, b.y);
     }
     const float2 bb = sb1[4 * j + t];
-    h1[j][0] = silu_fast(c[0] + bb.x); h1[j][1] = silu_fast(c[1] + bb.y);
-    h1[j][2] = silu_fast(c[2] + bb.x); h1[j][3] = silu_fast(c[3] + bb.y);
+    const float2 lo = silu_fast2(c[0], c[1], bb), hi = silu_fast2(c[2], c[3], bb);
+    h1[j][0] = pack_bf16(lo.x, lo.y);
+    h1[j][1] = pack_bf16(hi.x, hi.y);
   }
   ea = 0.f;
   eb = 0.f;
-#pragma unroll
+#pragma unroll 2
   for (int j = 0; j < 8; ++j) {
     float c[4] = {0.f, 0.f, 0.f, 0.f};
     const int n = 8 * j + g;
 #pragma unroll
     for (int kt = 0; kt < 4; ++kt) {
-      const uint32_t a[4] = {pack_bf16(h1[2 * kt][0], h1[2 * kt][1]), pack_bf16(h1[2 * kt][2], h1[2 * kt][3]),
-                             pack_bf16(h1[2 * kt + 1][0], h1[2 * kt + 1][1]),
-                             pack_bf16(h1[2 * kt + 1][2], h1[2 * kt + 1][3])};
+      const uint32_t a[4] = {h1[2 * kt][0], h1[2 * kt][1], h1[2 * kt + 1][0], h1[2 * kt + 1][1]};
       const uint2 b = sW2[(n * MLP_S2 + 8 * kt + 2 * t) >> 1];
       mma16816(c, a, b.x, b.y);
     }
     const float2 bb = sb2[4 * j + t];
     const float2 ww = sw3[4 * j + t];
-    ea = __fmaf_rn(silu_fast(c[0] + bb.x), ww.x, ea);
-    ea = __fmaf_rn(silu_fast(c[1] + bb.y), ww.y, ea);
-    eb = __fmaf_rn(silu_fast(c[2] + bb.x), ww.x, eb);
-    eb = __fmaf_rn(silu_fast(c[3] + bb.y), ww.y, eb);
+    const float2 lo = silu_fast2(c[0], c[1], bb), hi = silu_fast2(c[2], c[3], bb);
+    ea = __fmaf_rn(lo.x, ww.x, ea);
+    ea = __fmaf_rn(lo.y, ww.y, ea);
+    eb = __fmaf_rn(hi.x, ww.x, eb);
+    eb = __fmaf_rn(hi.y, ww.y, eb);
   }
   ea += __shfl_xor_sync(0xffffffffu, ea, 1);
   ea += __shfl_xor_sync(0xffffffffu, ea, 2);

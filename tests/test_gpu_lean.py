@@ -138,3 +138,48 @@ def test_grand_lean_path(gpu, oracle, kw, lanes, max_N, box):
         for g, o in zip(b.translation_counts(w), ow.translation_counts()):
             np.testing.assert_array_equal(g, o)
         np.testing.assert_allclose(b.state(w), ow.state(), atol=1e-11)
+
+
+@pytest.mark.parametrize("n,kw", [
+    (13, dict(method="sad", energy_bin=0.002, min_allowed=-38.0, max_allowed=-5.0)),
+    (33, dict(method="sad", energy_bin=0.3, max_allowed=50.0)),
+    (40, dict(method="samc", energy_bin=0.3, min_allowed=-120.0, max_allowed=2.0)),
+    (20, dict(method="samc", energy_bin=5.0, max_allowed=0.0)),
+    (13, dict(method="wl", energy_bin=2.0, max_allowed=0.0)),
+    (64, dict(method="sad", energy_bin=0.2, max_allowed=0.0))], ids=lambda k: k if isinstance(k, int) else k["method"])
+def test_delayed_acceptance_lean_path(gpu, oracle, n, kw):
+    """Both stages of delayed-acceptance moves, taken by the oracle from the traced energies
+    and surrogate changes."""
+    W, seed, R, plain, runs = 5, 8, 1.05 * n ** (1 / 3), 2400, (2500, 37, 1000)
+    okw = dict(METHOD_KW[kw["method"]], **{k: v for k, v in kw.items() if k != "method"},
+               target_rate=0.5, translation_scale=0.1)
+    confs = lj_configs(oracle, n, R, range(60, 60 + W))
+    b = gpu.Batch(gpu.make_config(gpu.LJ, W, n, e_lo=-6.0 * n - 6, e_hi=kw["max_allowed"] + 6.0, seed=seed,
+                                  lanes_per_walker=32, **okw), [(n, R, (0, 0, 0))] * W)
+    b.upload(confs)
+    b.initialize()
+    E0 = b.energies()
+    total = plain + sum(runs)
+    b.set_trace(total)
+    b.surrogate_init(seed=2, ring_capacity=4096)
+    for _ in range(6):
+        b.run(plain // 6)
+        b.surrogate_collect()
+    b.surrogate_train(60, batch=64, lr=2e-3, seed=4)
+    for k in runs:
+        b.run_da(k, refresh_interval=512)
+    out_of_range = b.status() & gpu.ST_BIN_RANGE
+    assert not out_of_range.all()
+    for w in range(W):
+        if out_of_range[w]:
+            continue  # the reference would have grown its bins
+        e1, e2 = b.trace(w, total)
+        ds = b.trace_ds(w, total)
+        ow = oracle.Walker(oracle.make_config(oracle.LJ, n, radius=R, seed=seed, walker=w, e0=float(E0[w]), **okw),
+                           confs[w])
+        d1, m1 = ow.run_override(e1[:plain], e2[:plain])
+        d2, m2 = ow.run_override_da(e1[plain:], e2[plain:], ds[plain:])
+        assert m1 == 0 and m2 == 0 and max(d1, d2) < REPLAY_REL, (w, m1, m2, d1, d2)
+        assert_bins_equal(b.bins(w), ow.bins(), label=f"walker {w}")
+        assert_scalars_equal(b.scalars(w), ow.scalars(), label=f"walker {w}")
+        np.testing.assert_allclose(b.state(w), ow.state(), atol=1e-11)
