@@ -86,64 +86,78 @@ __host__ __device__ constexpr int mlp_wword(int n, int w, int stride) {
   return n * stride + (w >> 3) * 8 + 2 * (w & 3) + ((w >> 2) & 1);
 }
 
-// Surrogate energies of 16 rows (one warp): A fragments of G from a row-major bf16 tile
-// in shared memory (32 bf16 = 16 words per row), weights in the mlp_wword layout and biases
+// Surrogate energies of T tiles of 16 rows (one warp): A fragments of G from a row-major bf16
+// tile in shared memory (32 bf16 = 16 words per row), weights in the mlp_wword layout and biases
 // as float pairs in shared memory, SiLU in its tanh form (silu_fast2).  Rows g and g+8 of
-// the tile end in ea / eb (in the quad's lane t == 0 and the others alike).
-template <int RW>  // 32-bit words between consecutive rows of the tile
+// tile m end in ea[m] / eb[m] (in the quad's lane t == 0 and the others alike).  The tiles share
+// each weight fragment that is loaded.
+template <int RW, int T>  // RW: 32-bit words between consecutive rows
 __device__ __forceinline__ void mlp16(const uint32_t* gtile, const uint2* sW1, const uint2* sW2,
                                       const float2* sb1, const float2* sb2, const float2* sw3,
-                                      float b3, float& ea, float& eb) {
+                                      float b3, float (&ea)[T], float (&eb)[T]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  uint32_t aG[2][4];
+  uint32_t aG[T][2][4];
 #pragma unroll
-  for (int kt = 0; kt < 2; ++kt) {
-    aG[kt][0] = gtile[g * RW + 8 * kt + t];
-    aG[kt][1] = gtile[(g + 8) * RW + 8 * kt + t];
-    aG[kt][2] = gtile[g * RW + 8 * kt + 4 + t];
-    aG[kt][3] = gtile[(g + 8) * RW + 8 * kt + 4 + t];
-  }
-  uint32_t h1[8][2];  // units 8 j + 2 t, + 1 of rows g and g + 8, as layer 2 takes them
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    const int n = 8 * j + g;
+  for (int m = 0; m < T; ++m) {
+    const uint32_t* p = gtile + 16 * m * RW;
 #pragma unroll
     for (int kt = 0; kt < 2; ++kt) {
-      const uint2 b = sW1[(n * MLP_S1 + 8 * kt + 2 * t) >> 1];
-      mma16816(c, aG[kt], b.x, b.y);
+      aG[m][kt][0] = p[g * RW + 8 * kt + t];
+      aG[m][kt][1] = p[(g + 8) * RW + 8 * kt + t];
+      aG[m][kt][2] = p[g * RW + 8 * kt + 4 + t];
+      aG[m][kt][3] = p[(g + 8) * RW + 8 * kt + 4 + t];
     }
-    const float2 bb = sb1[4 * j + t];
-    const float2 lo = silu_fast2(c[0], c[1], bb), hi = silu_fast2(c[2], c[3], bb);
-    h1[j][0] = pack_bf16(lo.x, lo.y);
-    h1[j][1] = pack_bf16(hi.x, hi.y);
   }
-  ea = 0.f;
-  eb = 0.f;
+  uint32_t h1[T][8][2];  // units 8 j + 2 t, + 1 of rows g and g + 8, as layer 2 takes them
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int n = 8 * j + g;
+    const uint2 w0 = sW1[(n * MLP_S1 + 2 * t) >> 1], w1 = sW1[(n * MLP_S1 + 8 + 2 * t) >> 1];
+    const float2 bb = sb1[4 * j + t];
+#pragma unroll
+    for (int m = 0; m < T; ++m) {
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      mma16816(c, aG[m][0], w0.x, w0.y);
+      mma16816(c, aG[m][1], w1.x, w1.y);
+      const float2 lo = silu_fast2(c[0], c[1], bb), hi = silu_fast2(c[2], c[3], bb);
+      h1[m][j][0] = pack_bf16(lo.x, lo.y);
+      h1[m][j][1] = pack_bf16(hi.x, hi.y);
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < T; ++m) ea[m] = eb[m] = 0.f;
 #pragma unroll 2
   for (int j = 0; j < 8; ++j) {
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
     const int n = 8 * j + g;
+    uint2 b[4];
 #pragma unroll
-    for (int kt = 0; kt < 4; ++kt) {
-      const uint32_t a[4] = {h1[2 * kt][0], h1[2 * kt][1], h1[2 * kt + 1][0], h1[2 * kt + 1][1]};
-      const uint2 b = sW2[(n * MLP_S2 + 8 * kt + 2 * t) >> 1];
-      mma16816(c, a, b.x, b.y);
-    }
+    for (int kt = 0; kt < 4; ++kt) b[kt] = sW2[(n * MLP_S2 + 8 * kt + 2 * t) >> 1];
     const float2 bb = sb2[4 * j + t];
     const float2 ww = sw3[4 * j + t];
-    const float2 lo = silu_fast2(c[0], c[1], bb), hi = silu_fast2(c[2], c[3], bb);
-    ea = __fmaf_rn(lo.x, ww.x, ea);
-    ea = __fmaf_rn(lo.y, ww.y, ea);
-    eb = __fmaf_rn(hi.x, ww.x, eb);
-    eb = __fmaf_rn(hi.y, ww.y, eb);
+#pragma unroll
+    for (int m = 0; m < T; ++m) {
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kt = 0; kt < 4; ++kt) {
+        const uint32_t a[4] = {h1[m][2 * kt][0], h1[m][2 * kt][1], h1[m][2 * kt + 1][0], h1[m][2 * kt + 1][1]};
+        mma16816(c, a, b[kt].x, b[kt].y);
+      }
+      const float2 lo = silu_fast2(c[0], c[1], bb), hi = silu_fast2(c[2], c[3], bb);
+      ea[m] = __fmaf_rn(lo.x, ww.x, ea[m]);
+      ea[m] = __fmaf_rn(lo.y, ww.y, ea[m]);
+      eb[m] = __fmaf_rn(hi.x, ww.x, eb[m]);
+      eb[m] = __fmaf_rn(hi.y, ww.y, eb[m]);
+    }
   }
-  ea += __shfl_xor_sync(0xffffffffu, ea, 1);
-  ea += __shfl_xor_sync(0xffffffffu, ea, 2);
-  eb += __shfl_xor_sync(0xffffffffu, eb, 1);
-  eb += __shfl_xor_sync(0xffffffffu, eb, 2);
-  ea += b3;
-  eb += b3;
+#pragma unroll
+  for (int m = 0; m < T; ++m) {
+    ea[m] += __shfl_xor_sync(0xffffffffu, ea[m], 1);
+    ea[m] += __shfl_xor_sync(0xffffffffu, ea[m], 2);
+    eb[m] += __shfl_xor_sync(0xffffffffu, eb[m], 1);
+    eb[m] += __shfl_xor_sync(0xffffffffu, eb[m], 2);
+    ea[m] += b3;
+    eb[m] += b3;
+  }
 }
 
 }  // namespace dev
