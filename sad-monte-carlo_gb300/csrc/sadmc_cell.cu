@@ -140,17 +140,18 @@ struct WcaGrandShared {
 
 template <int LPW>
 __global__ void __launch_bounds__(128) wca_grand_kernel(GrandLaunch m) {
-  constexpr int WPW = 32 / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   __shared__ WcaGrandShared<LPW> sh[4];
   const int lane = threadIdx.x & 31;
   const int group = lane / LPW, glane = lane % LPW;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
+  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   WcaGrandShared<LPW>& S = sh[threadIdx.x >> 5];
   CellProposal& P = S.prop[group];
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
   GrandBook<LPW> bk;
   bk.load(m, w, glane, gmask, wr);
@@ -438,10 +439,12 @@ cudaError_t launch_cell_energy(const WalkerCore* cores, const CellSys& s, int n_
 namespace sadmc {
 cudaError_t launch_wca_grand_move(const GrandLaunch& m, cudaStream_t st) {
   const int lpw = m.lanes == 8 || m.lanes == 16 ? m.lanes : 32;
-  const int warps = (m.n_walkers + (32 / lpw) - 1) / (32 / lpw);
-  if (lpw == 8) dev::wca_grand_kernel<8><<<(warps + 3) / 4, 128, 0, st>>>(m);
-  else if (lpw == 16) dev::wca_grand_kernel<16><<<(warps + 3) / 4, 128, 0, st>>>(m);
-  else dev::wca_grand_kernel<32><<<(warps + 3) / 4, 128, 0, st>>>(m);
+  GrandLaunch ms = m;
+  ms.walkers_per_warp = spread_walkers(m.n_walkers, 32 / lpw);
+  const int warps = (m.n_walkers + ms.walkers_per_warp - 1) / ms.walkers_per_warp;
+  if (lpw == 8) dev::wca_grand_kernel<8><<<(warps + 3) / 4, 128, 0, st>>>(ms);
+  else if (lpw == 16) dev::wca_grand_kernel<16><<<(warps + 3) / 4, 128, 0, st>>>(ms);
+  else dev::wca_grand_kernel<32><<<(warps + 3) / 4, 128, 0, st>>>(ms);
   return cudaGetLastError();
 }
 }  // namespace sadmc

@@ -355,14 +355,15 @@ struct CellOps {
 // it.
 template <int LPW, int KIND>
 __global__ void __launch_bounds__(128, 1) cell_descent_kernel(MoveLaunch m, CellSys s) {
-  constexpr int WPW = 32 / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;
+  if (warp * wpw >= m.n_walkers) return;
   const int group = lane / LPW, glane = lane % LPW;
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
 
   __shared__ BucketScan sbs[128 / LPW];
@@ -609,16 +610,18 @@ struct alignas(16) CellShared {
 // their index in that order, evaluated one per lane, and then summed in it.
 template <int LPW, int KIND, int FAM>
 __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys s) {
-  constexpr int WPW = 32 / LPW, ROUNDS = (27 + LPW - 1) / LPW;
+  constexpr int ROUNDS = (27 + LPW - 1) / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   extern __shared__ __align__(16) unsigned char cell_smem[];
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;
+  if (warp * wpw >= m.n_walkers) return;
   CellShared<LPW, KIND>& S = reinterpret_cast<CellShared<LPW, KIND>*>(cell_smem)[threadIdx.x >> 5];
   const int group = lane / LPW, glane = lane % LPW;
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
   CellProposal& P = S.prop[group];
 
@@ -982,13 +985,15 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
 namespace dev {
 template <int LPW, int KIND, int FAM>
 cudaError_t launch_cell(const MoveLaunch& m, const CellSys& s, cudaStream_t st) {
-  const int warps = (m.n_walkers + (32 / LPW) - 1) / (32 / LPW);
+  MoveLaunch ms = m;
+  ms.walkers_per_warp = spread_walkers(m.n_walkers, 32 / LPW);
+  const int warps = (m.n_walkers + ms.walkers_per_warp - 1) / ms.walkers_per_warp;
   int wpb = m.warps_per_block >= 1 && m.warps_per_block <= 4 ? m.warps_per_block : 4;
   constexpr size_t per = sizeof(CellShared<LPW, KIND>);
   constexpr int most = (int)(227 * 1024 / per) < 4 ? (int)(227 * 1024 / per) : 4;  // warps a block can hold
   static_assert(most >= 1, "a warp's tables fit a block");
   if (m.descent) {
-    cell_descent_kernel<LPW, KIND><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(m, s);
+    cell_descent_kernel<LPW, KIND><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(ms, s);
     return cudaGetLastError();
   }
   if (wpb > most) wpb = most;
@@ -1004,7 +1009,7 @@ cudaError_t launch_cell(const MoveLaunch& m, const CellSys& s, cudaStream_t st) 
     if (e != cudaSuccess) return e;
     if (device >= 0 && device < 64) attr[device].store(true, std::memory_order_release);
   }
-  cell_move_kernel<LPW, KIND, FAM><<<(warps + wpb - 1) / wpb, 32 * wpb, wpb * per, st>>>(m, s);
+  cell_move_kernel<LPW, KIND, FAM><<<(warps + wpb - 1) / wpb, 32 * wpb, wpb * per, st>>>(ms, s);
   return cudaGetLastError();
 }
 }  // namespace dev

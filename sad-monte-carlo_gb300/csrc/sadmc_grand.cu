@@ -16,6 +16,7 @@
 #include "sadmc_fh.cuh"
 #include "sadmc_grand.h"
 #include "sadmc_grand_book.cuh"
+#include "sadmc_launch.h"
 #include "sadmc_lj_walker.cuh"
 #include "sadmc_rng.cuh"
 
@@ -46,16 +47,17 @@ struct GrandWarpShared {
 // 31 atoms, 4096 moves, 20.9 -> 12.1 ms.
 template <int LPW, int APL>
 __global__ void __launch_bounds__(128) lj_grand_kernel(GrandLaunch m) {
-  constexpr int WPW = 32 / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   __shared__ GrandWarpShared<LPW, APL> sh[4];
   const int lane = threadIdx.x & 31;
   const int group = lane / LPW, glane = lane % LPW;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
+  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   GrandWarpShared<LPW, APL>& S = sh[threadIdx.x >> 5];
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
   GrandBook<LPW> bk;
   bk.load(m, w, glane, gmask, wr);
@@ -261,8 +263,10 @@ __global__ void grand_init_kernel(GrandLaunch m) {
 
 #define SADMC_GRAND_CASE(L, A)                                                          \
   if (m.lanes == L && m.np == L * A) {                                                  \
-    const int warps = (m.n_walkers + (32 / L) - 1) / (32 / L);                          \
-    dev::lj_grand_kernel<L, A><<<(warps + 3) / 4, 128, 0, st>>>(m);                     \
+    GrandLaunch ms = m;                                                                 \
+    ms.walkers_per_warp = spread_walkers(m.n_walkers, 32 / L);                          \
+    const int warps = (m.n_walkers + ms.walkers_per_warp - 1) / ms.walkers_per_warp;    \
+    dev::lj_grand_kernel<L, A><<<(warps + 3) / 4, 128, 0, st>>>(ms);                    \
     return cudaGetLastError();                                                          \
   }
 

@@ -68,6 +68,7 @@ struct GrandLaunch {
   int* cell_atoms;
   uint64_t* words;       // [walker][cells] each bucket's count and first atoms (cell_word)
   int cell_cap, bucket;
+  int walkers_per_warp;  // set by the launchers (spread_walkers)
   double box[3];
   int nc[3];
   double r_cut;

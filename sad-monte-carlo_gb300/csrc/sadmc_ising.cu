@@ -21,14 +21,15 @@ namespace dev {
 
 template <int LPW, int FAM>
 __global__ void __launch_bounds__(128) ising_move_kernel(MoveLaunch m, IsingSys s) {
-  constexpr int WPW = 32 / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;
+  if (warp * wpw >= m.n_walkers) return;
   const int group = lane / LPW, glane = lane % LPW;
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
   __shared__ RateTable rates[4];
   __shared__ double gammas[4][LPW > 1 ? 128 : 1];
@@ -134,19 +135,21 @@ __global__ void ising_energy_kernel(IsingSys s, int n_walkers, double* out) {
 constexpr size_t kIsingStageMax = 200 * 1024;
 
 cudaError_t launch_ising_move(const MoveLaunch& m, const IsingSys& s, int lpw, cudaStream_t st) {
-  const int wpw = 32 / lpw;
+  const int wpw = spread_walkers(m.n_walkers, 32 / lpw);
   const int warps = (m.n_walkers + wpw - 1) / wpw;
+  MoveLaunch ms = m;
+  ms.walkers_per_warp = wpw;
   const int wpb = m.warps_per_block >= 1 && m.warps_per_block <= 4 ? m.warps_per_block : 4;
   const int blocks = (warps + wpb - 1) / wpb;
   if (lpw == 1) {
-    if (m.method == M_SAD && !m.descent) dev::ising_move_kernel<1, M_SAD><<<blocks, 32 * wpb, 0, st>>>(m, s);
-    else dev::ising_move_kernel<1, dev::FAM_ANY><<<blocks, 32 * wpb, 0, st>>>(m, s);
+    if (m.method == M_SAD && !m.descent) dev::ising_move_kernel<1, M_SAD><<<blocks, 32 * wpb, 0, st>>>(ms, s);
+    else dev::ising_move_kernel<1, dev::FAM_ANY><<<blocks, 32 * wpb, 0, st>>>(ms, s);
   } else if (lpw == 32) {
     // a lone walker per warp: its moves as a serial chain on one lane when its planes and
     // spins fit in shared memory
     if (!m.descent && ising_chain_bytes(m.P.nbins, s.L) <= kIsingStageMax)
       return launch_ising_chain(m, s, kIsingStageMax, st);
-    dev::ising_move_kernel<32, dev::FAM_ANY><<<blocks, 32 * wpb, 0, st>>>(m, s);
+    dev::ising_move_kernel<32, dev::FAM_ANY><<<blocks, 32 * wpb, 0, st>>>(ms, s);
   } else {
     return cudaErrorInvalidConfiguration;
   }

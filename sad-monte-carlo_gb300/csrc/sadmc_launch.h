@@ -25,6 +25,7 @@ struct MoveLaunch {
   uint64_t descent_limit;  // maximum descent proposals per walker
   double descent_max;      // max_allowed_energy the descent aims below
   int warps_per_block;     // 1, 2 or 4 (kernels are bounded to 128 threads)
+  int walkers_per_warp;    // set by the launchers that spread few walkers (spread_walkers)
   int method;              // the configured method (selects a specialised kernel)
 };
 
@@ -115,5 +116,14 @@ cudaError_t launch_numerics_check(uint64_t n, uint64_t seed, unsigned long long*
 cudaError_t launch_draws(int system, uint32_t n, uint64_t seed, uint32_t walker, uint64_t t0,
                          int count, uint32_t stream_pair, uint32_t* idx2, float* g3, double* u,
                          cudaStream_t st);
+
+// Walkers of a warp that has room for `most`: as few as keep the warps at one per scheduler (4 per SM).
+// The walkers of a warp advance in step, so that one on the general path stops all of them, and a
+// scheduler without a warp is idle: 4096 Ising walkers of 32 x 32, 8192 moves, 27.4 ms with 32 a warp
+// (128 warps), 19.6 with 8 (512), 20.0 with 4 (1024), 39.6 with 2; 1024 LJ31 walkers on 8 lanes
+// each, 24414 moves, 41.0 ms with 4 a warp (256 warps), 37.2 with 2, 36.7 with 1; 8192 LJ38
+// walkers on 2 lanes, 40.0 ms with 16 a warp (512 warps), 42.9 with 8 (1024).  The other groups
+// of the warp repeat the walkers' work.
+int spread_walkers(int n_walkers, int most);
 
 }  // namespace sadmc

@@ -38,14 +38,15 @@ namespace dev {
 // descent stream until E < max_allowed_energy.
 template <int LPW, int APL>
 __global__ void __launch_bounds__(128) lj_descent_kernel(MoveLaunch m, LjSys s) {
-  constexpr int WPW = 32 / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
+  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   const int group = lane / LPW, glane = lane % LPW;
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   WalkerCore c = m.cores[w];
   LjWalker<LPW, APL> lj;
   lj.set_radius2(s.radius2);
@@ -107,16 +108,17 @@ struct LjWarpShared {
 
 template <int LPW, int APL, int FAM>
 __global__ void __launch_bounds__(128) lj_move_kernel(MoveLaunch m, LjSys s) {
-  constexpr int WPW = 32 / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   __shared__ LjWarpShared<LPW, APL> sh[4];
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
+  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   LjWarpShared<LPW, APL>& S = sh[threadIdx.x >> 5];
   const int group = lane / LPW, glane = lane % LPW;
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
 
   Fh<LPW, FAM, BOOK_LEAN> fh;
@@ -278,9 +280,11 @@ __global__ void __launch_bounds__(128) lj_move_kernel(MoveLaunch m, LjSys s) {
 #define SADMC_LJ_CASE(L, A, F, D)                                                      \
   if (lpw == L && s.np == L * A) {                                                     \
     const int wpb = m.warps_per_block >= 1 && m.warps_per_block <= 4 ? m.warps_per_block : 4; \
-    const int warps = (m.n_walkers + (32 / L) - 1) / (32 / L);                         \
-    if constexpr (D) dev::lj_descent_kernel<L, A><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(m, s); \
-    else dev::lj_move_kernel<L, A, F><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(m, s); \
+    MoveLaunch ms = m;                                                                 \
+    ms.walkers_per_warp = spread_walkers(m.n_walkers, 32 / L);                         \
+    const int warps = (m.n_walkers + ms.walkers_per_warp - 1) / ms.walkers_per_warp;   \
+    if constexpr (D) dev::lj_descent_kernel<L, A><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(ms, s); \
+    else dev::lj_move_kernel<L, A, F><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, st>>>(ms, s); \
     return cudaGetLastError();                                                         \
   }
 #define SADMC_LJ_ALL_SHAPES(F, D)                                                      \

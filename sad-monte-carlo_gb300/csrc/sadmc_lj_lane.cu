@@ -64,16 +64,18 @@ struct LjLaneShared {
 
 template <int LPW, int NP, int FAM>
 __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
-  constexpr int WPW = 32 / LPW, APL = NP / LPW;
+  constexpr int APL = NP / LPW;
+  const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   extern __shared__ __align__(16) unsigned char lane_smem[];
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * WPW >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
+  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   LjLaneShared<LPW, NP>& S = reinterpret_cast<LjLaneShared<LPW, NP>*>(lane_smem)[threadIdx.x >> 5];
   const int group = lane / LPW, glane = lane % LPW;
-  int w = warp * WPW + group;
-  const bool wr = w < m.n_walkers;
-  if (!wr) w = m.n_walkers - 1;
+  // groups past the warp's walkers repeat those of the first ones without effect
+  int w = warp * wpw + (group & (wpw - 1));
+  const bool wr = group < wpw && w < m.n_walkers;
+  if (w >= m.n_walkers) w = m.n_walkers - 1;
   const unsigned gmask = group_mask<LPW>(group);
 
   Fh<LPW, FAM, BOOK_LEAN> fh;
@@ -233,7 +235,6 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
 
 template <int LPW, int NP, int FAM>
 cudaError_t launch_lane(const MoveLaunch& m, const LjSys& s, cudaStream_t st) {
-  constexpr int WPW = 32 / LPW;
   const int wpb = m.warps_per_block >= 1 && m.warps_per_block <= 4 ? m.warps_per_block : 1;
   const size_t bytes = (size_t)wpb * sizeof(LjLaneShared<LPW, NP>);
   // Larger than the default 48 KB for 64-atom walkers: the limit is raised once per device
@@ -248,8 +249,10 @@ cudaError_t launch_lane(const MoveLaunch& m, const LjSys& s, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     if (device >= 0 && device < 64) attr[device].store(true, std::memory_order_release);
   }
-  const int warps = (m.n_walkers + WPW - 1) / WPW;
-  lj_lane_kernel<LPW, NP, FAM><<<(warps + wpb - 1) / wpb, 32 * wpb, bytes, st>>>(m, s);
+  MoveLaunch ms = m;
+  ms.walkers_per_warp = spread_walkers(m.n_walkers, 32 / LPW);
+  const int warps = (m.n_walkers + ms.walkers_per_warp - 1) / ms.walkers_per_warp;
+  lj_lane_kernel<LPW, NP, FAM><<<(warps + wpb - 1) / wpb, 32 * wpb, bytes, st>>>(ms, s);
   return cudaGetLastError();
 }
 

@@ -337,5 +337,15 @@ cudaError_t launch_numerics_check(uint64_t n, uint64_t seed, unsigned long long*
   return cudaGetLastError();
 }
 
+int spread_walkers(int n_walkers, int most) {
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return most;
+  int k = most;
+  while (k > 1 && (n_walkers + k / 2 - 1) / (k / 2) <= 4 * sms) k /= 2;
+  return k;
+}
+
 }  // namespace sadmc
 

@@ -183,3 +183,49 @@ def test_delayed_acceptance_lean_path(gpu, oracle, n, kw):
         assert_bins_equal(b.bins(w), ow.bins(), label=f"walker {w}")
         assert_scalars_equal(b.scalars(w), ow.scalars(), label=f"walker {w}")
         np.testing.assert_allclose(b.state(w), ow.state(), atol=1e-11)
+
+
+@pytest.mark.parametrize("system,lanes", [("ising", 1), ("lj", 8), ("lj", 2), ("wca", 8), ("grand_lj", 8), ("grand_wca", 8)])
+def test_few_walkers_run_as_in_a_large_batch(gpu, oracle, system, lanes):
+    """A small batch has few walkers per warp, the rest of it repeating their work; a large one
+    fills its warps.  A walker's chain is the same."""
+    few, runs = 11, (700, 33)
+    many = 20000 if lanes == 1 else 11000 if lanes == 2 else 3000
+
+    def batch(W):
+        if system.startswith("grand"):
+            geo = dict(box=(4.5,) * 3) if system == "grand_wca" else dict(radius=2.5)
+            return gpu.GrandBatch(gpu.make_grand_config(W, 20, t0=500.0, energy_bin=0.5, max_allowed=10.0, e_lo=-90.0,
+                                                        e_hi=12.0, translation_scale=0.1, addremove_probability=0.2,
+                                                        seed=4, lanes_per_walker=lanes, **geo))
+        if system == "ising":
+            cfg = gpu.make_config(gpu.ISING, W, 8, e_lo=-140.0, e_hi=140.0, seed=4, lanes_per_walker=1,
+                                  **METHOD_KW["sad"], energy_bin=4.0)
+            geo, confs = (8, 0.0, (0, 0, 0)), [ising_spins(8, w % few) for w in range(W)]
+        else:
+            n, kind = (13, gpu.LJ) if system == "lj" else (24, gpu.WCA)
+            kw = dict(METHOD_KW["sad"], energy_bin=0.5, target_rate=0.5, translation_scale=0.1)
+            cfg = gpu.make_config(kind, W, n, e_lo=-60.0 if kind == gpu.LJ else -1.0, e_hi=1.0 if kind == gpu.LJ else 400.0,
+                                  max_allowed=0.0 if kind == gpu.LJ else 390.0, seed=4, lanes_per_walker=lanes, **kw)
+            if kind == gpu.LJ:
+                geo, pool = (n, 2.2, (0, 0, 0)), lj_configs(oracle, n, 2.2, range(40, 40 + few))
+            else:
+                geo = (n, 0.0, (4.0, 4.0, 4.0))
+                pool = [np.random.default_rng(w).permutation(np.stack(np.meshgrid(*[np.arange(3) * 1.3] * 3), -1)
+                                                             .reshape(-1, 3))[:n] for w in range(few)]
+            confs = [pool[w % few] for w in range(W)]
+        b = gpu.Batch(cfg, [geo] * W)
+        b.upload(confs)
+        b.initialize()
+        return b
+
+    a, b = batch(few), batch(many)
+    for k in runs:
+        a.run(k)
+        b.run(k)
+    for w in range(few):
+        x, y = a.bins(w), b.bins(w)
+        for k in x:
+            np.testing.assert_array_equal(x[k], y[k], err_msg=f"walker {w} {k}")
+        assert a.scalars(w) == b.scalars(w), w
+        np.testing.assert_array_equal(a.state(w), b.state(w))
