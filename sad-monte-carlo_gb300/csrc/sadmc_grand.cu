@@ -44,9 +44,10 @@ struct GrandWarpShared {
 // batch's moves (an add's position too), all kinds share one packed pair loop (an add has no
 // old position, a removal no new one), and an ordinary SAMC move takes the lean path.
 // Bound by the warp instructions of a step, with two warps per scheduler: 4096 walkers of up to
-// 31 atoms, 4096 moves, 20.9 -> 12.1 ms.
+// 31 atoms, 4096 moves, 20.9 -> 11.3 ms.  (Two blocks to an SM: left to itself the compiler keeps to
+// the 168 registers of three, 12.1 ms.)
 template <int LPW, int APL>
-__global__ void __launch_bounds__(128) lj_grand_kernel(GrandLaunch m) {
+__global__ void __launch_bounds__(128, 2) lj_grand_kernel(GrandLaunch m) {
   const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   __shared__ GrandWarpShared<LPW, APL> sh[4];
   const int lane = threadIdx.x & 31;

@@ -20,7 +20,9 @@ namespace sadmc {
 namespace dev {
 
 template <int LPW, int FAM>
-__global__ void __launch_bounds__(128) ising_move_kernel(MoveLaunch m, IsingSys s) {
+// (Two blocks to an SM: left to itself the compiler keeps to the 168 registers of three, 4096
+// walkers of 32 x 32, 8192 moves, 19.6 against 19.1 ms.)
+__global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingSys s) {
   const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);

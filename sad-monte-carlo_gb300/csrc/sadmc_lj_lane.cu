@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
   for (uint32_t it = 0; it < n_moves; ++it) {
     const int kb = (int)(it % LPW);
     if (kb == 0) {
-      d = draws_continuous(m.seed, (uint32_t)w, fh.c.moves + 1 + (uint64_t)glane, (uint32_t)n, 0u);
+      d = draws_continuous<true>(m.seed, (uint32_t)w, fh.c.moves + 1 + (uint64_t)glane, (uint32_t)n, 0u);
       displace();
     }
     const double2 rate = S.rate.get(it, fh.c.moves, lane);
