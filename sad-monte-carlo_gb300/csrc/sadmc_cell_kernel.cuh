@@ -116,13 +116,6 @@ struct CellWalker {
     }
     return e;
   }
-  // The same sum for atom i over all 27 subcells around its own.
-  template <class F>
-  __device__ double pair_sum64(int i, F f) const {
-    const int ci = cell_of[i];
-    return near_sum64(p[i], p[np + i], p[2 * np + i], ci / (nc[1] * nc[2]), (ci / nc[2]) % nc[1],
-                      ci % nc[2], i, f, 0, 1);
-  }
 };
 
 // potential_pressure (wca.rs:79-92): -r dV/dr / 2 for r < 2^(1/6), sigma = epsilon = 1.
@@ -532,9 +525,9 @@ __device__ __forceinline__ uint64_t cell_word(const int* list, int count) {
 __device__ __forceinline__ int word_count(uint64_t w) { return (int)(w >> 48); }
 __device__ __forceinline__ int word_atom(uint64_t w, int s) { return (int)(w >> (12 * s)) & 0xfff; }
 
-// CellWalker::pair_sum64 over the words, for an f that is 0 from the cutoff on: a binary32
-// screen with a margin leaves out the candidates that would add nothing (five in six), which
-// spares their FP64 distances.  Same order, same bits.
+// The FP64 sum of f(r^2) for atom i over the 27 subcells around its own, in the order of their
+// words, for an f that is 0 from the cutoff on: a binary32 screen with a margin leaves out the
+// candidates that would add nothing (five in six), which spares their FP64 distances.
 template <class F>
 __device__ double pair_sum64_screened(const CellWalker& cw, const uint64_t* words, int i, float reach, F f) {
   const double qx = cw.p[i], qy = cw.p[cw.np + i], qz = cw.p[2 * cw.np + i];
