@@ -16,7 +16,7 @@
 // sqrt(1/t) are tables in shared memory that all lanes fill, read back with one load each
 // instead of shuffles.  Measured on one GB300 (4096 LJ31 walkers, 8 lanes, SAD, past their
 // first 37 k moves): 990 -> 578 warp instructions per step, 3.53 -> 1.94 us; 1024 walkers
-// 3.17 -> 1.69 us.  The same walkers' first 12 k moves: 53.2 -> 37.8 ms.
+// 3.17 -> 1.54 us (1.69 with four walkers in a warp).  The same walkers' first 12 k moves: 53.2 -> 37.8 ms.
 //
 // Every resum_interval moves the energy
 // is replaced by an FP64 pair sum over the double-single positions (compute_energy,
