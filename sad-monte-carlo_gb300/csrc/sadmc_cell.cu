@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(128) wca_grand_kernel(GrandLaunch m) {
       P.nh[ax] = th; P.oh[ax] = fh;
       P.nl[ax] = (float)(tax - (double)th); P.ol[ax] = (float)(f - (double)fh);
     }
+    __syncwarp();  // the proposal is stored before any lane reads it: a vote orders no memory
     const unsigned bads = __ballot_sync(0xffffffffu, bad);
     bad = (bads & gmask) != 0;
     const float4 nh = *reinterpret_cast<const float4*>(P.nh), oh = *reinterpret_cast<const float4*>(P.oh),

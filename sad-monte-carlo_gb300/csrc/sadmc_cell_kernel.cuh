@@ -708,6 +708,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
         if (KIND == SYS_WCA) { P.nl[ax] = (float)(tax - (double)th); P.ol[ax] = (float)(f - (double)fhi); }
       }
     }
+    __syncwarp();  // the proposal is stored before any lane reads it: a vote orders no memory
     const unsigned bads = __ballot_sync(0xffffffffu, bad);
     bad = (bads & gmask) != 0;
     const float4 nh = *reinterpret_cast<const float4*>(P.nh), oh = *reinterpret_cast<const float4*>(P.oh);

@@ -1,0 +1,41 @@
+"""Memory ordering inside a warp, read from the kernels' sources (a race shows no fault on a
+run that happens to be in step).  Votes and shuffles order no memory: what one lane stores
+and another reads has a __syncwarp between."""
+import os
+import re
+
+import pytest
+
+from conftest import PKG
+
+
+def source(name):
+    """The file's text without comments."""
+    with open(os.path.join(PKG, "csrc", name)) as f:
+        return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", f.read(), flags=re.S))
+
+
+def kernel(name, function):
+    """The body of a __global__ function."""
+    text = source(name)
+    head = re.search(r"__global__[^;{]*?\b" + function + r"\(", text)
+    start = text.index("{", head.end())
+    depth = 0
+    for k in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[k], 0)
+        if depth == 0:
+            return text[start:k + 1]
+    raise AssertionError(function)
+
+
+CELL_KERNELS = [("sadmc_cell_kernel.cuh", "cell_move_kernel"), ("sadmc_cell.cu", "wca_grand_kernel")]
+
+
+@pytest.mark.parametrize("name,function", CELL_KERNELS)
+def test_proposal_is_stored_before_it_is_read(name, function):
+    """Three lanes of a group store the proposal, an axis each; all of them read it."""
+    body = kernel(name, function)
+    stores = [m.end() for m in re.finditer(r"\bP\.\w+(\[\w+\])+\s*=[^=]", body)]
+    reads = [m.start() for m in re.finditer(r"\(P\.\w+|= P\.\w+", body) if m.start() > max(stores)]
+    assert stores and reads
+    assert "__syncwarp()" in body[max(stores):min(reads)]
