@@ -351,6 +351,7 @@ __global__ void __launch_bounds__(128) wca_grand_kernel(GrandLaunch m) {
       m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
     }
     int r = bk.wl_method ? 2 : bk.lean_decide(m, possible, de, N2, u.y);
+    __syncwarp();  // every lane has read the proposed bin and bucket before one lane stores to it
     if (SADMC_RARE(r == 2)) {
       r = possible && bk.decide(m, E1, N1, E1 + (double)de, N2, translation, u.y) ? 1 : 0;
       bk.finish(m, t, E1, N1);

@@ -39,3 +39,13 @@ def test_proposal_is_stored_before_it_is_read(name, function):
     reads = [m.start() for m in re.finditer(r"\(P\.\w+|= P\.\w+", body) if m.start() > max(stores)]
     assert stores and reads
     assert "__syncwarp()" in body[max(stores):min(reads)]
+
+
+@pytest.mark.parametrize("name,function", [("sadmc_grand.cu", "lj_grand_kernel"), ("sadmc_cell.cu", "wca_grand_kernel")])
+def test_proposed_bin_is_read_before_it_is_stored(name, function):
+    """Every lane of a group reads the proposed bin's fields (and the bucket's word) to decide;
+    one lane of it then books the move in them."""
+    body = kernel(name, function)
+    decide, book = body.index("bk.lean_decide("), body.index("bk.lean_finish(")
+    assert decide < book
+    assert "__syncwarp()" in body[decide:book]
