@@ -145,16 +145,13 @@ __global__ void __launch_bounds__(128) wca_grand_kernel(GrandLaunch m) {
   const int lane = threadIdx.x & 31;
   const int group = lane / LPW, glane = lane % LPW;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   WcaGrandShared<LPW>& S = sh[threadIdx.x >> 5];
   CellProposal& P = S.prop[group];
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  if (group >= wpw || w >= m.n_walkers) return;  // the collectives are over the lanes that stay
   const unsigned gmask = group_mask<LPW>(group);
   GrandBook<LPW> bk;
-  bk.load(m, w, glane, gmask, wr);
+  bk.load(m, w, glane, gmask);
   bk.gtab = S.gamma + group * 4 * LPW;
   CellWalker cw;
   cw.np = m.np;
@@ -358,7 +355,7 @@ __global__ void __launch_bounds__(128) wca_grand_kernel(GrandLaunch m) {
     } else {
       bk.lean_finish(m, t, r == 1, de, N2, translation);
     }
-    if (r == 1 && wr) {
+    if (r == 1) {
       // ConfirmSystem::confirm (wca.rs:276-301) on the buckets
       if (glane == 0) {
         if (has_old && !stay) {  // `which` leaves its bucket

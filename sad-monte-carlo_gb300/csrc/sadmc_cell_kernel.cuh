@@ -351,17 +351,14 @@ __global__ void __launch_bounds__(128, 1) cell_descent_kernel(MoveLaunch m, Cell
   const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * wpw >= m.n_walkers) return;
   const int group = lane / LPW, glane = lane % LPW;
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  if (group >= wpw || w >= m.n_walkers) return;  // the collectives are over the lanes that stay
   const unsigned gmask = group_mask<LPW>(group);
 
   __shared__ BucketScan sbs[128 / LPW];
   Fh<LPW> fh;
-  fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
+  fh.load(m.cores, m.P, m.B, w, gmask, glane, true);
   CellWalker cw;
   cw.np = s.np;
   cw.bucket = s.bucket;
@@ -456,7 +453,7 @@ __global__ void __launch_bounds__(128, 1) cell_descent_kernel(MoveLaunch m, Cell
         pos = x > pos ? x : pos;
       }
       __syncwarp(gmask);
-      if (wr && pos >= 0) {
+      if (pos >= 0) {
         lo[pos] = lo[mo - 1];
         cw.cnt[p.old_c] = mo - 1;
         cw.atoms[(size_t)p.new_c * cw.bucket + p.new_count] = a;
@@ -464,10 +461,8 @@ __global__ void __launch_bounds__(128, 1) cell_descent_kernel(MoveLaunch m, Cell
         cw.cell_of[a] = p.new_c;
       }
     }
-    if (wr) {
-      cw.p[a] = p.tx; cw.p[s.np + a] = p.ty; cw.p[2 * s.np + a] = p.tz;
-      put_ds<KIND == SYS_WCA>(cw.p32, a, p.tx, p.ty, p.tz);
-    }
+    cw.p[a] = p.tx; cw.p[s.np + a] = p.ty; cw.p[2 * s.np + a] = p.tz;
+    put_ds<KIND == SYS_WCA>(cw.p32, a, p.tx, p.ty, p.tz);
     __syncwarp(gmask);
   };
 
@@ -509,7 +504,7 @@ __global__ void __launch_bounds__(128, 1) cell_descent_kernel(MoveLaunch m, Cell
     }
     fh.c.pad2 = steps;
     fh.c.pad1 = done ? 1 : 0;
-    if (wr && glane == 0) m.cores[w] = fh.c;  // the host re-sums E in FP64 afterwards
+    if (glane == 0) m.cores[w] = fh.c;  // the host re-sums E in FP64 afterwards
   }
 }
 
@@ -608,18 +603,15 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
   extern __shared__ __align__(16) unsigned char cell_smem[];
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * wpw >= m.n_walkers) return;
   CellShared<LPW, KIND>& S = reinterpret_cast<CellShared<LPW, KIND>*>(cell_smem)[threadIdx.x >> 5];
   const int group = lane / LPW, glane = lane % LPW;
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  if (group >= wpw || w >= m.n_walkers) return;  // the collectives are over the lanes that stay
   const unsigned gmask = group_mask<LPW>(group);
   CellProposal& P = S.prop[group];
 
   Fh<LPW, FAM, BOOK_LEAN> fh;
-  fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
+  fh.load(m.cores, m.P, m.B, w, gmask, glane, true);
   fh.gtab = S.gamma + group * 4 * LPW;
   fh.lean_sync();
   CellWalker cw;
@@ -663,7 +655,8 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
   for (uint32_t it = 0; it < n_moves; ++it) {
     const int kb = (int)(it % LPW);
     const uint64_t t = fh.c.moves + 1;
-    const double2 rate = S.rate.get(it, fh.c.moves, lane);
+    if ((it & 31u) == 0) S.rate.fill(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
+    const double2 rate = S.rate.v[it & 31u];
     if (kb == 0) {
       const Draws d = draws_continuous(m.seed, (uint32_t)w, t + (uint64_t)glane, (uint32_t)n, 0u);
       __syncwarp(gmask);
@@ -887,7 +880,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
         fh.c.status |= ST_CELL_OVERFLOW;
       }
     }
-    if (SADMC_RARE(m.trace && wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap)) {
+    if (SADMC_RARE(m.trace && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap)) {
       TraceRec r;
       r.e1 = fh.c.E;
       r.e2 = possible ? fh.c.E + (double)de : __longlong_as_double(0x7ff8000000000000ll);
@@ -917,7 +910,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
           pos = x > pos ? x : pos;
         }
         __syncwarp(gmask);
-        if (wr && glane == 0 && pos >= 0) {
+        if (glane == 0 && pos >= 0) {
           int* ln = cw.atoms + (size_t)new_c * cw.bucket;
           lo[pos] = lo[mo - 1];
           ln[new_count] = a;
@@ -928,8 +921,8 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
           words[new_c] = cell_word(ln, new_count + 1);
         }
       }
-      if (wr && glane < 3) cw.p[(size_t)ax * s.np + a] = tax;
-      if (wr && glane == 0) {
+      if (glane < 3) cw.p[(size_t)ax * s.np + a] = tax;
+      if (glane == 0) {
         if (KIND == SYS_WCA) {
           cw.p32[2 * a] = make_float4(nh.x, nh.y, nh.z, 0.0f);
           cw.p32[2 * a + 1] = make_float4(P.nl[0], P.nl[1], P.nl[2], 0.0f);
@@ -946,7 +939,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
       for (int i = glane; i < n; i += LPW)
         pv += pair_sum64_screened(cw, words, i, wsqr32 + 1e-3f, [&](double r2) { return wca_pressure64(r2, wsqr); });
       pv = group_sum<LPW>(pv, gmask);
-      if (wr && glane == 0) {
+      if (glane == 0) {
         const size_t k = (size_t)w * fh.nbins + fh.cur;
         m.B.ex_count[k] += 1;
         m.B.ex_total[k] += pv / (3.0 * (cw.L[0] * cw.L[1] * cw.L[2]));

@@ -75,6 +75,13 @@ __device__ __forceinline__ float rcp_hw(float x) {
   return r;
 }
 
+// The walkers of a warp that has room for wpw of them: they take its first lane groups, and the
+// lanes of the other groups leave the kernel, so that one group alone reads and writes a
+// walker's memory.  A mask that names lanes that have left is a mask of the others.
+__device__ __forceinline__ int warp_walkers(int n_walkers, int warp, int wpw) {
+  return min(wpw, n_walkers - warp * wpw);
+}
+
 template <int LPW>
 __device__ __forceinline__ unsigned group_mask(int group) {
   return LPW == 32 ? 0xffffffffu : (((1u << LPW) - 1u) << (group * LPW));

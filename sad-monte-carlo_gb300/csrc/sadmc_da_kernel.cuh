@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
     }
     if (refresh_every.tick()) refresh();
   }
-  lj.store(pw, s.np, true);
+  lj.store(pw, s.np);
   fh.store(m.cores, w);
   if (stats && lane == 0) {
     stats[2 * w] += screened_out;

@@ -183,7 +183,7 @@ struct Fh {
   // lane group
   unsigned gmask;
   int glane;
-  bool wr;  // stores enabled (false for padding groups past the last walker)
+  bool wr;  // stores enabled (the one-walker chain: on its deciding lane)
   // cached current bin (global index cur)
   int cur;
   double k_lnw, k_sE, k_sE2;
@@ -1231,20 +1231,21 @@ struct RecentScale {
   }
 };
 
-// sqrt(1/t) and 1 - sqrt(1/t) of 32 consecutive moves in a warp's shared memory: filled by
-// its 32 lanes (whose walkers share the move count), read with one load per move.
+// sqrt(1/t) and 1 - sqrt(1/t) of 32 consecutive moves in a warp's shared memory: filled by its
+// lanes (whose walkers share the move count), read with one load per move.
 struct RateTable {
   double2 v[32];  // x = sqrt(1/t), y = 1 - x (energy.rs:913)
-  // the factors of the it-th move of a launch, the moves counted before it; called by the
-  // whole warp
-  __device__ double2 get(uint32_t it, uint64_t moves, int lane) {
-    if ((it & 31u) == 0) {
-      const double r = sqrt(1.0 / (double)(moves + 1 + (uint64_t)lane));
-      __syncwarp();
-      v[lane] = make_double2(r, 1. - r);
-      __syncwarp();
+  // The factors of the 32 moves after `moves`; called by the warp's first `lanes` lanes, the
+  // others having left.  (Two at a time: a lone walker's lanes have several each, whose FP64
+  // chains then overlap.)
+  __device__ void fill(uint64_t moves, int lane, int lanes) {
+    __syncwarp();
+#pragma unroll 2
+    for (int k = lane; k < 32; k += lanes) {
+      const double r = sqrt(1.0 / (double)(moves + 1 + (uint64_t)k));
+      v[k] = make_double2(r, 1. - r);
     }
-    return v[it & 31u];
+    __syncwarp();
   }
 };
 

@@ -53,15 +53,12 @@ __global__ void __launch_bounds__(128, 2) lj_grand_kernel(GrandLaunch m) {
   const int lane = threadIdx.x & 31;
   const int group = lane / LPW, glane = lane % LPW;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   GrandWarpShared<LPW, APL>& S = sh[threadIdx.x >> 5];
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  if (group >= wpw || w >= m.n_walkers) return;  // the collectives are over the lanes that stay
   const unsigned gmask = group_mask<LPW>(group);
   GrandBook<LPW> bk;
-  bk.load(m, w, glane, gmask, wr);
+  bk.load(m, w, glane, gmask);
   bk.gtab = S.gamma + group * 4 * LPW;
   const float wall_r2f = __double2float_rn(m.radius2);
   float* pw = m.pos + (size_t)w * 6 * (size_t)m.np;
@@ -235,16 +232,14 @@ __global__ void __launch_bounds__(128, 2) lj_grand_kernel(GrandLaunch m) {
       bk.resummed(m, lj.energy64());
     }
   }
-  if (wr) {
 #pragma unroll
-    for (int k = 0; k < APL; ++k)
+  for (int k = 0; k < APL; ++k)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int j = glane + LPW * k;
-        pw[c * m.np + j] = S.at(c, 0, k, lane);
-        pw[(3 + c) * m.np + j] = S.at(c, 1, k, lane);
-      }
-  }
+    for (int c = 0; c < 3; ++c) {
+      const int j = glane + LPW * k;
+      pw[c * m.np + j] = S.at(c, 0, k, lane);
+      pw[(3 + c) * m.np + j] = S.at(c, 1, k, lane);
+    }
   bk.store(m.cores, w);
 }
 

@@ -24,7 +24,7 @@ struct GrandBook {
   unsigned gmask;
   double width, inv_width;
   bool wl_method;
-  bool wr, lead;  // a walker's group (not a padding one); its lane 0, which stores its results
+  bool lead;  // lane 0 of the group, which stores its results
   // u_choice53 > ar_thresh  <=>  u_choice53 * 2^-53 > addremove_prob (scaling by a power of
   // two is exact, and u is an integer: u > p 2^53 <=> u > floor(p 2^53))
   int64_t ar_thresh;
@@ -46,11 +46,10 @@ struct GrandBook {
   int wl_low;      // WL: visited bins whose WL count is at most lowest (-1: to be counted)
   double* gtab;    // SAMC's gamma of 4 LPW moves, in shared memory
 
-  __device__ void load(const GrandLaunch& m, int w, int glane_, unsigned gmask_, bool wr_ = true) {
+  __device__ void load(const GrandLaunch& m, int w, int glane_, unsigned gmask_) {
     c = m.cores[w];
     glane = glane_;
-    wr = wr_;
-    lead = glane_ == 0 && wr;
+    lead = glane_ == 0;
     gmask = gmask_;
     rows = m.rows;
     ncol = m.ncol;
@@ -129,7 +128,7 @@ struct GrandBook {
     for (int k = glane; k < total; k += LPW) {
       const int r = e_base + k / ncols, q = k % ncols;
       if (r >= old_lo && r < old_hi && q <= old_n) continue;
-      if (wr) visit[plane(r, q)] = c.fill_gen << 1;  // a new bin starts not visited
+      visit[plane(r, q)] = c.fill_gen << 1;  // a new bin starts not visited
     }
     __syncwarp(gmask);
     cur_row_ok = false;
@@ -243,7 +242,7 @@ struct GrandBook {
           c.lowest = wl_i;
           if (total > 1 && (double)c.lowest >= 0.8 * (double)c.total / num_states) {
             c.gamma *= 0.5;
-            for (int k = glane; wr && k < total; k += LPW) wlh[plane(c.e_base + k / ncols, k % ncols)] = 0;
+            for (int k = glane; k < total; k += LPW) wlh[plane(c.e_base + k / ncols, k % ncols)] = 0;
             c.total = 0;
             c.lowest = 0;
             __syncwarp(gmask);

@@ -29,15 +29,17 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (warp * wpw >= m.n_walkers) return;
   const int group = lane / LPW, glane = lane % LPW;
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  // a lane past the warp's walkers touches no walker's memory: it leaves the descent, and fills
+  // the rate table with the others between the moves
+  const bool own = group < wpw && w < m.n_walkers;
+  if (m.descent && !own) return;
   const unsigned gmask = group_mask<LPW>(group);
   __shared__ RateTable rates[4];
   __shared__ double gammas[4][LPW > 1 ? 128 : 1];
   Fh<LPW, FAM, BOOK_LEAN, true> fh;
-  fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
+  const uint64_t moves0 = m.cores[warp * wpw].moves;  // the walkers share it
+  if (own) fh.load(m.cores, m.P, m.B, w, gmask, glane, true);
   const int L = s.L;
   int8_t* S = s.spins + (size_t)w * (size_t)L * (size_t)L;
   if (m.descent) {
@@ -58,7 +60,7 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
         const int sij = S[i + j * L];
         const double e2 = fh.c.E - (double)(nt * sij * 2);
         if (fh.uni(e2 < fh.c.E)) {
-          if (wr) S[i + j * L] = (int8_t)(-sij);
+          S[i + j * L] = (int8_t)(-sij);
           if (LPW > 1) __syncwarp(gmask);
           fh.c.E = e2;
         }
@@ -69,49 +71,56 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
     }
     fh.c.pad2 = steps;
     fh.c.pad1 = done ? 1 : 0;
-    if (wr && glane == 0) m.cores[w] = fh.c;
+    if (glane == 0) m.cores[w] = fh.c;
     return;
   }
   RateTable& rt = rates[threadIdx.x >> 5];
-  fh.gtab = gammas[threadIdx.x >> 5] + (LPW > 1 ? group * 4 * LPW : 0);
-  fh.lean_sync();
   DrawCache<LPW, true> dc;
   dc.init();
+  if (own) {
+    fh.gtab = gammas[threadIdx.x >> 5] + (LPW > 1 ? group * 4 * LPW : 0);
+    fh.lean_sync();
+  }
   const uint32_t n_moves = (uint32_t)m.n_moves;
-  for (uint32_t it = 0; it < n_moves; ++it) {
-    const uint64_t t = fh.c.moves + 1;
-    const double2 rate = rt.get(it, fh.c.moves, lane);
-    fh.begin_move(rate.y);
-    const Draws d = dc.get(m.seed, (uint32_t)w, t, (uint32_t)L, gmask, glane);
-    const int i = (int)d.which, j = (int)d.j;
-    int jp = j + 1 == L ? 0 : j + 1, jm = j == 0 ? L - 1 : j - 1;
-    int ip = i + 1 == L ? 0 : i + 1, im = i == 0 ? L - 1 : i - 1;
-    const int site = i + j * L;
-    const int nt = S[i + jp * L] + S[i + jm * L] + S[ip + j * L] + S[im + j * L];
-    const int sij = S[site];
-    const float de = (float)(-(nt * sij * 2));  // exact: |de| <= 8
-    if (m.trace && wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
-      TraceRec r;
-      r.e1 = fh.c.E;
-      r.e2 = fh.c.E + (double)de;
-      m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
-    }
-    int r = fh.lean_decide(true, de, d.u53);
-    if (SADMC_RARE(r == 2)) {
-      r = fh.decide_de(true, de, d.u53, rate.x) ? 1 : 0;
-      fh.finish_move(r == 1);
-      fh.lean_sync();
-    } else {
-      const int old_cur = fh.cur;
-      if (r == 1) fh.lean_accept(de, rate.x);
-      fh.lean_finish(old_cur);
-    }
-    if (r == 1) {
-      if (wr) S[site] = (int8_t)(-sij);  // all lanes of the group store the same value
-      if (LPW > 1) __syncwarp(gmask);
+  for (uint32_t base = 0; base < n_moves; base += 32) {
+    rt.fill(moves0 + base, lane, 32);
+    const uint32_t end = own ? min(base + 32u, n_moves) : base;
+    for (uint32_t it = base; it < end; ++it) {
+      const uint64_t t = fh.c.moves + 1;
+      const double2 rate = rt.v[it - base];
+      fh.begin_move(rate.y);
+      const Draws d = dc.get(m.seed, (uint32_t)w, t, (uint32_t)L, gmask, glane);
+      const int i = (int)d.which, j = (int)d.j;
+      int jp = j + 1 == L ? 0 : j + 1, jm = j == 0 ? L - 1 : j - 1;
+      int ip = i + 1 == L ? 0 : i + 1, im = i == 0 ? L - 1 : i - 1;
+      const int site = i + j * L;
+      const int nt = S[i + jp * L] + S[i + jm * L] + S[ip + j * L] + S[im + j * L];
+      const int sij = S[site];
+      const float de = (float)(-(nt * sij * 2));  // exact: |de| <= 8
+      if (m.trace && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
+        TraceRec r;
+        r.e1 = fh.c.E;
+        r.e2 = fh.c.E + (double)de;
+        m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
+      }
+      int r = fh.lean_decide(true, de, d.u53);
+      if (SADMC_RARE(r == 2)) {
+        r = fh.decide_de(true, de, d.u53, rate.x) ? 1 : 0;
+        fh.finish_move(r == 1);
+        fh.lean_sync();
+      } else {
+        const int old_cur = fh.cur;
+        if (r == 1) fh.lean_accept(de, rate.x);
+        fh.lean_finish(old_cur);
+      }
+      if (r == 1) {
+        if (LPW > 1) __syncwarp(gmask);  // after every lane's reads
+        S[site] = (int8_t)(-sij);        // all lanes of the group store the same value
+        if (LPW > 1) __syncwarp(gmask);
+      }
     }
   }
-  fh.store(m.cores, w);
+  if (own) fh.store(m.cores, w);
 }
 
 // compute_energy (ising.rs:59-75): sum over sites of s * (s_down + s_right), exact.

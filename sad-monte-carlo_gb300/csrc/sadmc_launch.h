@@ -122,8 +122,8 @@ cudaError_t launch_draws(int system, uint32_t n, uint64_t seed, uint32_t walker,
 // scheduler without a warp is idle: 4096 Ising walkers of 32 x 32, 8192 moves, 27.4 ms with 32 a warp
 // (128 warps), 19.6 with 8 (512), 20.0 with 4 (1024), 39.6 with 2; 1024 LJ31 walkers on 8 lanes
 // each, 24414 moves, 41.0 ms with 4 a warp (256 warps), 37.2 with 2, 36.7 with 1; 8192 LJ38
-// walkers on 2 lanes, 40.0 ms with 16 a warp (512 warps), 42.9 with 8 (1024).  The other groups
-// of the warp repeat the walkers' work.
+// walkers on 2 lanes, 40.0 ms with 16 a warp (512 warps), 42.9 with 8 (1024).  The lanes of the
+// other groups leave the kernel.
 int spread_walkers(int n_walkers, int most);
 
 }  // namespace sadmc

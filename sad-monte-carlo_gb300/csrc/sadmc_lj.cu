@@ -42,7 +42,7 @@ __global__ void lj_plan_kernel(WalkerCore* cores, LjSys s, int w, int which, flo
   if (lane == 0) { out[0] = ok ? e2 : 0.0; out[1] = ok ? 1.0 : 0.0; }
   if (ok && confirm) {
     lj.put(which, tx, ty, tz);
-    lj.store(pw, s.np, true);
+    lj.store(pw, s.np);
     if (lane == 0) cores[w].E = e2;
   }
 }

@@ -41,12 +41,9 @@ __global__ void __launch_bounds__(128) lj_descent_kernel(MoveLaunch m, LjSys s) 
   const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   const int group = lane / LPW, glane = lane % LPW;
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  if (group >= wpw || w >= m.n_walkers) return;  // the collectives are over the lanes that stay
   WalkerCore c = m.cores[w];
   LjWalker<LPW, APL> lj;
   lj.set_radius2(s.radius2);
@@ -84,8 +81,8 @@ __global__ void __launch_bounds__(128) lj_descent_kernel(MoveLaunch m, LjSys s) 
   c.E = e64;
   if (!(e64 < m.descent_max)) c.status |= ST_DESCENT_FAILED;
   else c.status &= ~(uint32_t)ST_DESCENT_FAILED;
-  lj.store(pw, s.np, wr);
-  if (wr && glane == 0) m.cores[w] = c;
+  lj.store(pw, s.np);
+  if (glane == 0) m.cores[w] = c;
 }
 
 // What a warp keeps in shared memory: its walkers' positions, and tables filled ahead by all
@@ -114,17 +111,14 @@ __global__ void __launch_bounds__(128, 2) lj_move_kernel(MoveLaunch m, LjSys s) 
   __shared__ LjWarpShared<LPW, APL> sh[4];
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   LjWarpShared<LPW, APL>& S = sh[threadIdx.x >> 5];
   const int group = lane / LPW, glane = lane % LPW;
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  if (group >= wpw || w >= m.n_walkers) return;  // the collectives are over the lanes that stay
   const unsigned gmask = group_mask<LPW>(group);
 
   Fh<LPW, FAM, BOOK_LEAN> fh;
-  fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
+  fh.load(m.cores, m.P, m.B, w, gmask, glane, true);
   fh.gtab = S.gamma + group * 4 * LPW;
   fh.lean_sync();
   const int n = fh.c.n;
@@ -157,7 +151,8 @@ __global__ void __launch_bounds__(128, 2) lj_move_kernel(MoveLaunch m, LjSys s) 
       d = draws_continuous(m.seed, (uint32_t)w, fh.c.moves + 1 + (uint64_t)glane, (uint32_t)n, 0u);
       displace();
     }
-    const double2 rate = S.rate.get(it, fh.c.moves, lane);
+    if ((it & 31u) == 0) S.rate.fill(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
+    const double2 rate = S.rate.v[it & 31u];
     fh.begin_move(rate.y);
     // plan_move of lj.rs:365-374 and move_atom of lj.rs:86-105
     const int e = group * LPW + kb;
@@ -208,7 +203,7 @@ __global__ void __launch_bounds__(128, 2) lj_move_kernel(MoveLaunch m, LjSys s) 
     de = group_sum<LPW>(de, 0xffffffffu);  // the warp's walkers take their moves together
     if (SADMC_RARE(m.trace != nullptr)) {
       const uint64_t t = fh.c.moves;
-      if (wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
+      if (glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
         TraceRec r;
         r.e1 = fh.c.E;
         r.e2 = possible ? fh.c.E + (double)de : __longlong_as_double(0x7ff8000000000000ll);
@@ -262,16 +257,14 @@ __global__ void __launch_bounds__(128, 2) lj_move_kernel(MoveLaunch m, LjSys s) 
       fh.lean_sync();
     }
   }
-  if (wr) {
 #pragma unroll
-    for (int k = 0; k < APL; ++k)
+  for (int k = 0; k < APL; ++k)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int j = glane + LPW * k;
-        pw[c * s.np + j] = S.at(c, 0, k, lane);
-        pw[(3 + c) * s.np + j] = S.at(c, 1, k, lane);
-      }
-  }
+    for (int c = 0; c < 3; ++c) {
+      const int j = glane + LPW * k;
+      pw[c * s.np + j] = S.at(c, 0, k, lane);
+      pw[(3 + c) * s.np + j] = S.at(c, 1, k, lane);
+    }
   fh.store(m.cores, w);
 }
 

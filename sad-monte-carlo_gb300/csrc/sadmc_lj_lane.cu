@@ -69,22 +69,20 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
   extern __shared__ __align__(16) unsigned char lane_smem[];
   const int lane = threadIdx.x & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (warp * wpw >= m.n_walkers) return;  // whole warp is padding (warp-uniform)
   LjLaneShared<LPW, NP>& S = reinterpret_cast<LjLaneShared<LPW, NP>*>(lane_smem)[threadIdx.x >> 5];
   const int group = lane / LPW, glane = lane % LPW;
-  // groups past the warp's walkers repeat those of the first ones without effect
-  int w = warp * wpw + (group & (wpw - 1));
-  const bool wr = group < wpw && w < m.n_walkers;
-  if (w >= m.n_walkers) w = m.n_walkers - 1;
+  const int w = warp * wpw + group;
+  if (group >= wpw || w >= m.n_walkers) return;  // the collectives are over the lanes that stay
   const unsigned gmask = group_mask<LPW>(group);
 
   Fh<LPW, FAM, BOOK_LEAN> fh;
-  fh.load(m.cores, m.P, m.B, w, gmask, glane, wr);
+  fh.load(m.cores, m.P, m.B, w, gmask, glane, true);
   fh.gtab = S.gamma + group * 4 * LPW;
   fh.lean_sync();
   const int n = fh.c.n;
   const float wall_r2f = __double2float_rn(s.radius2);
   float* pw = s.pos + (size_t)w * 6 * (size_t)NP;
+#pragma unroll 4
   for (int k = 0; k < APL; ++k)
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -93,9 +91,7 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
       S.at(c, 1, k, lane) = pw[(3 + c) * NP + j];
     }
   // the slot pairs that hold atoms of any walker of the warp
-  int pairs = (n + 2 * LPW - 1) / (2 * LPW);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) pairs = max(pairs, __shfl_xor_sync(0xffffffffu, pairs, o));
+  const int pairs = __reduce_max_sync(0xffffffffu, (n + 2 * LPW - 1) / (2 * LPW));
 
   DS sc = ds_from_double(fh.c.tscale);
   Every resum;
@@ -117,7 +113,8 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
       d = draws_continuous<true>(m.seed, (uint32_t)w, fh.c.moves + 1 + (uint64_t)glane, (uint32_t)n, 0u);
       displace();
     }
-    const double2 rate = S.rate.get(it, fh.c.moves, lane);
+    if ((it & 31u) == 0) S.rate.fill(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
+    const double2 rate = S.rate.v[it & 31u];
     fh.begin_move(rate.y);
     // plan_move of lj.rs:365-374 and move_atom of lj.rs:86-105: the energy change summed in
     // binary32 over the walker's lanes
@@ -157,7 +154,7 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
     const float de = group_sum<LPW>(dn - dold, 0xffffffffu);
     if (SADMC_RARE(m.trace != nullptr)) {
       const uint64_t t = fh.c.moves;
-      if (wr && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
+      if (glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
         TraceRec r;
         r.e1 = fh.c.E;
         r.e2 = possible ? fh.c.E + (double)de : __longlong_as_double(0x7ff8000000000000ll);
@@ -221,15 +218,14 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
       fh.lean_sync();
     }
   }
-  if (wr) {
-    for (int k = 0; k < APL; ++k)
+#pragma unroll 4
+  for (int k = 0; k < APL; ++k)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int j = glane + LPW * k;
-        pw[c * NP + j] = S.at(c, 0, k, lane);
-        pw[(3 + c) * NP + j] = S.at(c, 1, k, lane);
-      }
-  }
+    for (int c = 0; c < 3; ++c) {
+      const int j = glane + LPW * k;
+      pw[c * NP + j] = S.at(c, 0, k, lane);
+      pw[(3 + c) * NP + j] = S.at(c, 1, k, lane);
+    }
   fh.store(m.cores, w);
 }
 

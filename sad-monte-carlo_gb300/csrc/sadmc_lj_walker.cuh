@@ -60,8 +60,7 @@ struct LjWalker {
       z[k] = DS{p[2 * np + j], p[5 * np + j]};
     }
   }
-  __device__ void store(float* p, int np, bool wr) const {
-    if (!wr) return;
+  __device__ void store(float* p, int np) const {
 #pragma unroll
     for (int k = 0; k < APL; ++k) {
       int j = glane + LPW * k;

@@ -49,3 +49,21 @@ def test_proposed_bin_is_read_before_it_is_stored(name, function):
     decide, book = body.index("bk.lean_decide("), body.index("bk.lean_finish(")
     assert decide < book
     assert "__syncwarp()" in body[decide:book]
+
+
+SPREAD_KERNELS = [("sadmc_lj_kernel.cuh", "lj_descent_kernel"), ("sadmc_lj_kernel.cuh", "lj_move_kernel"),
+                  ("sadmc_lj_lane.cu", "lj_lane_kernel"), ("sadmc_ising.cu", "ising_move_kernel"),
+                  ("sadmc_cell_kernel.cuh", "cell_descent_kernel"), ("sadmc_cell_kernel.cuh", "cell_move_kernel"),
+                  ("sadmc_grand.cu", "lj_grand_kernel"), ("sadmc_cell.cu", "wca_grand_kernel")]
+
+
+@pytest.mark.parametrize("name,function", SPREAD_KERNELS)
+def test_one_lane_group_to_a_walker(name, function):
+    """A lane group without a walker of its own must not run another group's walker: that one
+    stores to the planes, spins and lists which the copy would read, with nothing between."""
+    body = kernel(name, function)
+    assert re.search(r"\bw = warp \* wpw \+ group;", body)
+    assert "n_walkers - 1" not in body
+    load = re.search(r"\w\.load\(m|= m\.cores\[w\]", body).start()
+    assert re.search(r"if \(group >= wpw \|\| w >= m\.n_walkers\) return;", body[:load]) or re.search(
+        r"own = group < wpw && w < m\.n_walkers;.*if \(m\.descent && !own\) return;.*if \(own\) f$", body[:load], re.S)
