@@ -312,6 +312,9 @@ struct Fh {
   __device__ void sync() {
     if (LPW > 1) __syncwarp(gmask);
   }
+  // The one lane of the group that counts in memory (a value that every lane holds is stored by
+  // all of them alike).
+  __device__ bool leads() const { return wr && (LPW == 1 || glane == 0); }
   // Lane 0's value of a predicate for the whole lane group.  Every branch that leads to a
   // group collective (__syncwarp, shuffles) takes its predicate through here, so the
   // lanes of a group always reach the same collectives.
@@ -1003,7 +1006,7 @@ struct Fh {
     if (SUMS) {
       k_sE += c.E;
       k_sE2 += E2;  // E2 == E * E (set_E)
-    } else if (wr && (LPW == 1 || glane == 0)) {
+    } else if (leads()) {
       atomicAdd(&sE[cur], c.E);
       atomicAdd(&sE2[cur], E2);
     }
@@ -1024,7 +1027,8 @@ struct Fh {
   }
   __device__ void mark_visited() {
     k_stamp = c.fill_gen;
-    if (wr) { stamp[cur] = c.fill_gen; rt[cur] = rt[cur] + 1; }
+    if (wr) stamp[cur] = c.fill_gen;
+    if (leads()) rt[cur] = rt[cur] + 1;
   }
 
   // energy.rs:514-761
@@ -1117,7 +1121,7 @@ struct Fh {
   __device__ void wl_update() {  // energy.rs:638-752
     if (uni(c.has_min_gamma && c.gamma < c.min_gamma)) {  // production run
       int k = c.wl_lo + (cur - c.b_lo);
-      if (k >= c.wl_lo && k <= c.wl_hi) { if (wr) wlh[k] = wlh[k] + 1; }
+      if (k >= c.wl_lo && k <= c.wl_hi) { if (leads()) wlh[k] = wlh[k] + 1; }
       else c.status |= ST_BIN_RANGE;
       return;
     }
@@ -1159,7 +1163,9 @@ struct Fh {
       len_w = c.wl_hi - c.wl_lo + 1;
     }
     const int k = c.wl_lo + (cur - c.b_lo);
-    wl_count(k, wlh[k] + 1);
+    const uint64_t h = wlh[k] + 1;
+    sync();  // read by every lane before any stores it
+    wl_count(k, h);
   }
   // The stage histogram's new count h in plane bin k, and the flatness test
   // (energy.rs:700-752).

@@ -67,3 +67,22 @@ def test_one_lane_group_to_a_walker(name, function):
     load = re.search(r"\w\.load\(m|= m\.cores\[w\]", body).start()
     assert re.search(r"if \(group >= wpw \|\| w >= m\.n_walkers\) return;", body[:load]) or re.search(
         r"own = group < wpw && w < m\.n_walkers;.*if \(m\.descent && !own\) return;.*if \(own\) f$", body[:load], re.S)
+
+
+@pytest.mark.parametrize("name", ["sadmc_fh.cuh", "sadmc_grand_book.cuh"])
+def test_one_lane_counts_in_memory(name):
+    """A read-modify-write of a plane by all lanes of a group counts once only if they stay in
+    step."""
+    text = source(name)
+    steps = [m for m in re.finditer(r"\b(rt|wlh|tr_att|tr_acc)\[(?:[^\[\]]|\[\w+\])+\] (\+= 1|= \1\[)", text)]
+    assert steps
+    for m in steps:
+        assert re.search(r"if \((leads\(\)|lead)\) (\{[^}]*)?$", text[:m.start()]), m.group()
+
+
+def test_stage_count_is_read_before_it_is_stored():
+    """The general path's Wang-Landau update: every lane reads the bin's stage count, and stores
+    the next one."""
+    update = source("sadmc_fh.cuh").split("void wl_update()")[1].split("void wl_count(")[0]
+    read, count = update.rindex("wlh[k]"), update.rindex("wl_count(")
+    assert "sync();" in update[read:count]
