@@ -887,6 +887,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
       m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
     }
     int r = fh.lean_decide(possible, de, u53);
+    __syncwarp();  // the proposed bin is read by every lane before any stores to it
     if (SADMC_RARE(r == 2)) {
       r = fh.decide_de(possible, de, u53, rate.x) ? 1 : 0;
       fh.finish_move(r == 1);

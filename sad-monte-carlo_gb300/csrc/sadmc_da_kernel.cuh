@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
     }
     bool rej1, acc;
     const int r = fh.lean_delayed(possible, de, des, d.u53, u2, rej1);
+    __syncwarp();  // the proposed bin is read by every lane before any stores to it
     if (SADMC_RARE(r == 2)) {
       const double lnw_cur = fh.lnw_current();
       const double lnw_til = fh.lnw_at(e1 + (double)des);

@@ -315,11 +315,13 @@ struct Fh {
   // The one lane of the group that counts in memory (a value that every lane holds is stored by
   // all of them alike).
   __device__ bool leads() const { return wr && (LPW == 1 || glane == 0); }
-  // Lane 0's value of a predicate for the whole lane group.  Every branch that leads to a
-  // group collective (__syncwarp, shuffles) takes its predicate through here, so the
-  // lanes of a group always reach the same collectives.
   // the method: a compile-time constant in a specialised kernel (dead paths vanish)
   __device__ int kind() const { return FAM >= 0 ? FAM : (int)c.kind; }
+  // Lane 0's value of a predicate for the whole lane group, for the general path's branches
+  // that lead to a group collective (__syncwarp, shuffles), so that the lanes of a group reach
+  // the same ones.  The kernels' branch between the lean path and this one is taken by each lane on its
+  // own result: the lanes hold equal state, read equal proposals and planes (stores and reads of a
+  // plane are a barrier apart), and so agree.
   __device__ bool uni(bool x) const {
     if (LPW == 1) return x;
     return __shfl_sync(gmask, (int)x, 0, LPW) != 0;
@@ -596,6 +598,7 @@ struct Fh {
     double e2 = 0.0;
     bool have = false;
     const bool accepted = uni(!rejects(possible, de, u53, has_first, lnw_first, e2, have));
+    sync();  // the proposed bin is read by every lane before any stores to it
     if (accepted) {
       if (c.kind != M_DESCENT) { c.accepted += 1; if (!SPLIT) c.acc_rate += rs; }
       set_E(have ? e2 : c.E + f2d(de));

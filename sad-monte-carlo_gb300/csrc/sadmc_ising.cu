@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
         m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
       }
       int r = fh.lean_decide(true, de, d.u53);
+      if (LPW > 1) __syncwarp();  // the proposed bin is read by every lane before any stores to it
       if (SADMC_RARE(r == 2)) {
         r = fh.decide_de(true, de, d.u53, rate.x) ? 1 : 0;
         fh.finish_move(r == 1);

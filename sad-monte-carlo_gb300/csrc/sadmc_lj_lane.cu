@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
       }
     }
     int r = fh.lean_decide(possible, de, u53);
+    if (LPW > 1) __syncwarp();  // the proposed bin is read by every lane before any stores to it
     if (SADMC_RARE(r == 2)) {
       r = fh.decide_de(possible, de, u53, rate.x) ? 1 : 0;
       fh.finish_move(r == 1);

@@ -86,3 +86,16 @@ def test_stage_count_is_read_before_it_is_stored():
     update = source("sadmc_fh.cuh").split("void wl_update()")[1].split("void wl_count(")[0]
     read, count = update.rindex("wlh[k]"), update.rindex("wl_count(")
     assert "sync();" in update[read:count]
+
+
+@pytest.mark.parametrize("name,function", [
+    ("sadmc_lj_kernel.cuh", "lj_move_kernel"), ("sadmc_lj_lane.cu", "lj_lane_kernel"), ("sadmc_ising.cu", "ising_move_kernel"),
+    ("sadmc_cell_kernel.cuh", "cell_move_kernel"), ("sadmc_da_kernel.cuh", "lj_da_kernel")])
+def test_lean_decision_reads_before_the_booking_stores(name, function):
+    """The lean decision reads the proposed bin's stamp and stage count on every lane; the
+    booking stores them (the general path's likewise, inside decide_de)."""
+    body = kernel(name, function)
+    decide, book = re.search(r"fh\.lean_(decide|delayed)\(", body).start(), body.index("fh.decide_de(")
+    assert decide < book and re.search(r"__syncwarp\(\);.*if \(SADMC_RARE\(r == 2\)\)", body[decide:book], re.S)
+    general = source("sadmc_fh.cuh").split("bool decide_de(")[1].split("bool rejects(")[0]
+    assert "sync();" in general[general.index("rejects("):]
