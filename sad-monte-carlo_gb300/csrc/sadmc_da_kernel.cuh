@@ -249,7 +249,8 @@ __global__ void __launch_bounds__(32 * DA_WPB) lj_da_kernel(MoveLaunch m, LjSys 
   rsb.init();
   DrawCache<32, false> dc;
   dc.init();
-  uint64_t u2_all = 0, u2_t0 = ~0ull;  // the second-stage uniforms of 32 moves
+  // the second-stage uniforms of the 32 moves from u2_t0 on (none yet: the first move draws)
+  uint64_t u2_all = 0, u2_t0 = fh.c.moves + 1 - 32;
   DS sc = ds_from_double(fh.c.tscale);
   uint64_t screened_out = 0, exact_evals = 0;
   Every resum, refresh_every;
