@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys
   for (uint32_t it = 0; it < n_moves; ++it) {
     const int kb = (int)(it % LPW);
     const uint64_t t = fh.c.moves + 1;
-    if ((it & 31u) == 0) S.rate.fill(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
+    if (SADMC_RARE((it & 31u) == 0)) S.rate.fill<2>(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
     const double2 rate = S.rate.v[it & 31u];
     if (kb == 0) {
       const Draws d = draws_continuous(m.seed, (uint32_t)w, t + (uint64_t)glane, (uint32_t)n, 0u);

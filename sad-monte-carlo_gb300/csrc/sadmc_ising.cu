@@ -82,43 +82,41 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
     fh.lean_sync();
   }
   const uint32_t n_moves = (uint32_t)m.n_moves;
-  for (uint32_t base = 0; base < n_moves; base += 32) {
-    rt.fill(moves0 + base, lane, 32);
-    const uint32_t end = own ? min(base + 32u, n_moves) : base;
-    for (uint32_t it = base; it < end; ++it) {
-      const uint64_t t = fh.c.moves + 1;
-      const double2 rate = rt.v[it - base];
-      fh.begin_move(rate.y);
-      const Draws d = dc.get(m.seed, (uint32_t)w, t, (uint32_t)L, gmask, glane);
-      const int i = (int)d.which, j = (int)d.j;
-      int jp = j + 1 == L ? 0 : j + 1, jm = j == 0 ? L - 1 : j - 1;
-      int ip = i + 1 == L ? 0 : i + 1, im = i == 0 ? L - 1 : i - 1;
-      const int site = i + j * L;
-      const int nt = S[i + jp * L] + S[i + jm * L] + S[ip + j * L] + S[im + j * L];
-      const int sij = S[site];
-      const float de = (float)(-(nt * sij * 2));  // exact: |de| <= 8
-      if (m.trace && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
-        TraceRec r;
-        r.e1 = fh.c.E;
-        r.e2 = fh.c.E + (double)de;
-        m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
-      }
-      int r = fh.lean_decide(true, de, d.u53);
-      if (LPW > 1) __syncwarp();  // the proposed bin is read by every lane before any stores to it
-      if (SADMC_RARE(r == 2)) {
-        r = fh.decide_de(true, de, d.u53, rate.x) ? 1 : 0;
-        fh.finish_move(r == 1);
-        fh.lean_sync();
-      } else {
-        const int old_cur = fh.cur;
-        if (r == 1) fh.lean_accept(de, rate.x);
-        fh.lean_finish(old_cur);
-      }
-      if (r == 1) {
-        if (LPW > 1) __syncwarp(gmask);  // after every lane's reads
-        S[site] = (int8_t)(-sij);        // all lanes of the group store the same value
-        if (LPW > 1) __syncwarp(gmask);
-      }
+  for (uint32_t it = 0; it < n_moves; ++it) {
+    if (SADMC_RARE((it & 31u) == 0)) rt.fill<1>(moves0 + it, lane, 32);
+    if (!own) continue;
+    const uint64_t t = fh.c.moves + 1;
+    const double2 rate = rt.v[it & 31u];
+    fh.begin_move(rate.y);
+    const Draws d = dc.get(m.seed, (uint32_t)w, t, (uint32_t)L, gmask, glane);
+    const int i = (int)d.which, j = (int)d.j;
+    int jp = j + 1 == L ? 0 : j + 1, jm = j == 0 ? L - 1 : j - 1;
+    int ip = i + 1 == L ? 0 : i + 1, im = i == 0 ? L - 1 : i - 1;
+    const int site = i + j * L;
+    const int nt = S[i + jp * L] + S[i + jm * L] + S[ip + j * L] + S[im + j * L];
+    const int sij = S[site];
+    const float de = (float)(-(nt * sij * 2));  // exact: |de| <= 8
+    if (m.trace && glane == 0 && t > m.trace_t0 && t - m.trace_t0 <= m.trace_cap) {
+      TraceRec r;
+      r.e1 = fh.c.E;
+      r.e2 = fh.c.E + (double)de;
+      m.trace[(size_t)w * m.trace_cap + (t - m.trace_t0 - 1)] = r;
+    }
+    int r = fh.lean_decide(true, de, d.u53);
+    if (LPW > 1) __syncwarp();  // the proposed bin is read by every lane before any stores to it
+    if (SADMC_RARE(r == 2)) {
+      r = fh.decide_de(true, de, d.u53, rate.x) ? 1 : 0;
+      fh.finish_move(r == 1);
+      fh.lean_sync();
+    } else {
+      const int old_cur = fh.cur;
+      if (r == 1) fh.lean_accept(de, rate.x);
+      fh.lean_finish(old_cur);
+    }
+    if (r == 1) {
+      if (LPW > 1) __syncwarp(gmask);  // after every lane's reads
+      S[site] = (int8_t)(-sij);        // all lanes of the group store the same value
+      if (LPW > 1) __syncwarp(gmask);
     }
   }
   if (own) fh.store(m.cores, w);
