@@ -1246,9 +1246,11 @@ struct RecentScale {
 struct RateTable {
   double2 v[32];  // x = sqrt(1/t), y = 1 - x (energy.rs:913)
   // The factors of the 32 moves after `moves`; called by the warp's first `lanes` lanes, the
-  // others having left.  Lanes of a warp that is not full have several each, WAYS at a time so
-  // that their FP64 chains overlap.  (A loop over a variable number of them, unrolled by the
-  // compiler, divides by it: 4096 fresh LJ31 walkers 70.4 against 68.4 ms.)
+  // others having left.  Lanes of a warp that is not full have several each, one at a time (WAYS 1)
+  // or two whose FP64 chains overlap, whichever leaves the kernel around it quicker: LJ for SAD one
+  // (4096 fresh LJ31 walkers 64.9 against 67.1 ms, 64 walkers 22.4 against 22.7), LJ for the other
+  // methods two (4096 walkers, WL, 4096 moves, 9.9 against 10.5 ms), lane kernel one (8192 LJ38
+  // walkers, 8192 moves, 33.0 against 33.5 ms).
   template <int WAYS>
   __device__ void fill(uint64_t moves, int lane, int lanes) {
     auto rate = [&](int k) { return sqrt(1.0 / (double)(moves + 1 + (uint64_t)k)); };

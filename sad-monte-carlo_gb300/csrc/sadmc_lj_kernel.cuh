@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128, 2) lj_move_kernel(MoveLaunch m, LjSys s) 
       d = draws_continuous(m.seed, (uint32_t)w, fh.c.moves + 1 + (uint64_t)glane, (uint32_t)n, 0u);
       displace();
     }
-    if (SADMC_RARE((it & 31u) == 0)) S.rate.fill<2>(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
+    if (SADMC_RARE((it & 31u) == 0)) S.rate.fill<FAM == M_SAD ? 1 : 2>(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
     const double2 rate = S.rate.v[it & 31u];
     fh.begin_move(rate.y);
     // plan_move of lj.rs:365-374 and move_atom of lj.rs:86-105

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(128) lj_lane_kernel(MoveLaunch m, LjSys s) {
       d = draws_continuous<true>(m.seed, (uint32_t)w, fh.c.moves + 1 + (uint64_t)glane, (uint32_t)n, 0u);
       displace();
     }
-    if (SADMC_RARE((it & 31u) == 0)) S.rate.fill<4>(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
+    if (SADMC_RARE((it & 31u) == 0)) S.rate.fill<1>(fh.c.moves, lane, LPW * warp_walkers(m.n_walkers, warp, wpw));
     const double2 rate = S.rate.v[it & 31u];
     fh.begin_move(rate.y);
     // plan_move of lj.rs:365-374 and move_atom of lj.rs:86-105: the energy change summed in
