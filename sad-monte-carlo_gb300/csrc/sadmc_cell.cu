@@ -6,6 +6,7 @@
 
 namespace sadmc {
 cudaError_t launch_cell_move_wl(const MoveLaunch& m, const CellSys& s, int lpw, cudaStream_t st);
+cudaError_t launch_cell_move_general(const MoveLaunch& m, const CellSys& s, int lpw, cudaStream_t st);
 cudaError_t launch_cell_move_samc(const MoveLaunch& m, const CellSys& s, int lpw, cudaStream_t st);
 namespace dev {
 
@@ -409,7 +410,8 @@ __global__ void __launch_bounds__(128) wca_grand_kernel(GrandLaunch m) {
 cudaError_t launch_cell_move(const MoveLaunch& m, const CellSys& s, int lpw, cudaStream_t st) {
   if (m.method == M_WL) return launch_cell_move_wl(m, s, lpw, st);
   if (m.method == M_SAMC) return launch_cell_move_samc(m, s, lpw, st);
-  SADMC_CELL_ALL_SHAPES(dev::FAM_ANY)
+  if (general_method(m.method)) return launch_cell_move_general(m, s, lpw, st);
+  SADMC_CELL_ALL_SHAPES(M_SAD)
   return cudaErrorInvalidConfiguration;
 }
 

@@ -589,13 +589,13 @@ struct alignas(16) CellShared {
   typename std::conditional<KIND == SYS_WCA, CellPairs, CellNoPairs>::type pairs[32 / LPW];
 };
 
-// The move kernel.  FAM: the method it is specialised for, or FAM_ANY (the method each walker
-// holds).  A lane takes whole subcells (k = lane, lane + LPW, ... of the 27), whose words and
-// atoms' positions it requests together, so that a query costs two loads in sequence; a
-// proposal that stays in its subcell, the common case, reads its neighbourhood once for both
-// positions.  The square well counts contacts in any order.  The WCA sum keeps the order in
-// which each lane took every LPW-th candidate: pairs that reach the cutoff are collected with
-// their index in that order, evaluated one per lane, and then summed in it.
+// The move kernel.  FAM: the method it is specialised for, or FAM_GENERAL.  A lane takes
+// whole subcells (k = lane, lane + LPW, ...  of the 27), whose words and atoms' positions it
+// requests together, so that a query costs two loads in sequence; a proposal that stays in
+// its subcell, the common case, reads its neighbourhood once for both positions.  The square
+// well counts contacts in any order.  The WCA sum keeps the order in which each lane took
+// every LPW-th candidate: pairs that reach the cutoff are collected with their index in that
+// order, evaluated one per lane, and then summed in it.
 template <int LPW, int KIND, int FAM>
 __global__ void __launch_bounds__(128, 1) cell_move_kernel(MoveLaunch m, CellSys s) {
   constexpr int ROUNDS = (27 + LPW - 1) / LPW;

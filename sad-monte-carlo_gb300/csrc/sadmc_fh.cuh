@@ -149,8 +149,13 @@ __device__ __forceinline__ double sad_gamma_value(double p, uint64_t tF, uint64_
 }
 
 // FAM: the method a kernel is specialised for (M_SAD, ...), or FAM_ANY for the kind held
-// in each walker's state (WL and 1/t-WL, whose walkers switch to SAMC at run time).
+// in each walker's state (methods without an instance of their own).
 constexpr int FAM_ANY = -1;
+// FAM_GENERAL: as FAM_ANY, for the methods without a lean path (canonical; 1/t-WL until its
+// walkers switch), whose moves must not pay for an attempt at it.  The test in front of the
+// attempt has a kernel of its own because it costs the other methods' (4096 LJ31 walkers, 8 lanes,
+// 4096 moves: canonical 12.9 -> 11.8 ms with it, WL 9.87 -> 10.2 and SAMC 8.56 -> 8.94).
+constexpr int FAM_GENERAL = -2;
 
 // MODE: how the bookkeeping is divided.
 //  BOOK_FULL   everything here;
@@ -702,6 +707,10 @@ struct Fh {
   // estimate e2f = Ef + de is within 2 B 2.5e-7 of e2 (see decide_de); the thresholds take
   // 4e-7, which also covers their own rounding.
   __device__ void lean_sync() {
+    if (FAM == FAM_GENERAL) {
+      lean_off = kind() != M_SAD && kind() != M_SAMC && kind() != M_WL;
+      if (lean_off) return;
+    }
     const float B = fmaxf(fmaxf(fabsf(cminf), fabsf(cmaxf)), fabsf(Ef)), u = 4.0e-7f;
     // Integer energies that binary32 holds, with bin edges it holds at a power-of-two spacing:
     // the estimates are exact, and so are the comparisons with a threshold it holds.  (An odd
@@ -734,8 +743,7 @@ struct Fh {
     maxSf = f32_trunc(c.max_S);
     ddB = fabsf(maxSf) * 6.0e-7f + 1e-30f;
     cls = 0;
-    lean_off = (kind() != M_SAD && kind() != M_SAMC && kind() != M_WL) || binB > 0.25f || !(ddB < 0.2f) ||
-               (float)(c.b_hi - c.b_lo) > 4.0e6f;
+    lean_off = (kind() != M_SAD && kind() != M_SAMC && kind() != M_WL) || binB > 0.25f || !(ddB < 0.2f) || (float)(c.b_hi - c.b_lo) > 4.0e6f;
     if (kind() == M_SAD) {
       lean_off = lean_off || inverted;
       const float thif = f32_trunc(c.too_hi);
@@ -800,6 +808,7 @@ struct Fh {
   }
   template <bool FIRST>
   __device__ int lean_test(bool possible, float de, uint64_t u53, float a, float dd, float dmax) {
+    if (FAM == FAM_GENERAL && lean_off) return 2;
     const float e2f = Ef + de;
     const bool ordinary = e2f > in_lo && e2f < in_hi;
     const bool oob = (e2f > out_hi && de > tinyB) || (e2f < out_lo && de < -tinyB);
@@ -832,7 +841,7 @@ struct Fh {
     const bool rej = uf > __fmaf_rn(e32, mt, e32), acc = uf + (1.0f / 16777216.0f) < __fmaf_rn(-e32, mt, e32);
     const bool small = fabsf(de) <= tinyB && de != 0.0f;  // binary32 subnormals among them
     const bool decided = oob || (ordinary && !edge && !small && dd < 0.25f && (acc || rej));
-    if (SADMC_RARE(lean_off)) return 2;
+    if (FAM != FAM_GENERAL && SADMC_RARE(lean_off)) return 2;
     if (!possible || !(fabsf(de) <= 3.0e38f)) return 0;
     return decided ? (acc && !oob ? 1 : 0) : 2;
   }
@@ -1255,7 +1264,13 @@ struct RateTable {
   __device__ void fill(uint64_t moves, int lane, int lanes) {
     auto rate = [&](int k) { return sqrt(1.0 / (double)(moves + 1 + (uint64_t)k)); };
     __syncwarp();
-    if (lanes == 32) {
+    if constexpr (WAYS == 1) {
+#pragma unroll 1
+      for (int k = lane; k < 32; k += lanes) {
+        const double r = rate(k);
+        v[k] = make_double2(r, 1. - r);
+      }
+    } else if (lanes == 32) {
       const double r = rate(lane);
       v[lane] = make_double2(r, 1. - r);
     } else {

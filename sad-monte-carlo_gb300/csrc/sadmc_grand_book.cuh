@@ -313,6 +313,7 @@ struct GrandBook {
   // 1 accepted, 0 rejected, 2: the move is for decide() and finish().  (E, N) -> (E + de, n2).
   __device__ int lean_decide(const GrandLaunch& m, bool possible, float de, int n2, uint64_t u53) {
     if (SADMC_RARE(lean_stale)) lean_sync(m);
+    if (SADMC_RARE(lean_off)) return 2;
     const float e2f = Ef + de;
     const bool ordinary = e2f > in_lo && e2f < in_hi && n2 <= c.max_N_ref;
     const bool oob = (e2f > out_hi && de > tinyB) || (e2f < out_lo && de < -tinyB);
@@ -330,7 +331,6 @@ struct GrandBook {
     const float uf = (float)(uint32_t)(u53 >> 29) * (1.0f / 16777216.0f);
     const bool rej = uf > __fmaf_rn(e32, mt, e32), acc = uf + (1.0f / 16777216.0f) < __fmaf_rn(-e32, mt, e32);
     const bool small = fabsf(de) <= tinyB && de != 0.0f;
-    if (SADMC_RARE(lean_off)) return 2;
     if (!possible) return 0;
     return oob ? 0 : (ordinary && !edge && !small && (acc || rej) ? (acc ? 1 : 0) : 2);
   }

@@ -154,6 +154,7 @@ cudaError_t launch_ising_move(const MoveLaunch& m, const IsingSys& s, int lpw, c
   const int blocks = (warps + wpb - 1) / wpb;
   if (lpw == 1) {
     if (m.method == M_SAD && !m.descent) dev::ising_move_kernel<1, M_SAD><<<blocks, 32 * wpb, 0, st>>>(ms, s);
+    else if (general_method(m.method)) dev::ising_move_kernel<1, dev::FAM_GENERAL><<<blocks, 32 * wpb, 0, st>>>(ms, s);
     else dev::ising_move_kernel<1, dev::FAM_ANY><<<blocks, 32 * wpb, 0, st>>>(ms, s);
   } else if (lpw == 32) {
     // a lone walker per warp: its moves as a serial chain on one lane when its planes and

@@ -604,7 +604,8 @@ cudaError_t launch_ising_chain(const MoveLaunch& m, const IsingSys& s, size_t ma
   }
   const size_t bytes = dev::ising_chain_bytes(m.P.nbins, s.L);
   if (bytes > max_bytes) return cudaErrorInvalidConfiguration;
-  return dev::launch_chain<dev::FAM_ANY>(m, s, bytes, max_bytes, st);
+  return general_method(m.method) ? dev::launch_chain<dev::FAM_GENERAL>(m, s, bytes, max_bytes, st)
+                                  : dev::launch_chain<dev::FAM_ANY>(m, s, bytes, max_bytes, st);
 }
 
 }  // namespace sadmc

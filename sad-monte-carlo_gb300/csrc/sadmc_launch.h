@@ -117,6 +117,10 @@ cudaError_t launch_draws(int system, uint32_t n, uint64_t seed, uint32_t walker,
                          int count, uint32_t stream_pair, uint32_t* idx2, float* g3, double* u,
                          cudaStream_t st);
 
+// The methods whose moves have no lean path (FAM_GENERAL): canonical, and 1/t-WL until its walkers
+// switch themselves to SAMC.
+inline bool general_method(int method) { return method == M_CANONICAL || method == M_INV_T_WL; }
+
 // Walkers of a warp that has room for `most`: as few as keep the warps at one per scheduler (4 per SM).
 // The walkers of a warp advance in step, so that one on the general path stops all of them, and a
 // scheduler without a warp is idle: 4096 Ising walkers of 32 x 32, 8192 moves, 27.4 ms with 32 a warp

@@ -5,6 +5,7 @@
 #include "sadmc_lj_kernel.cuh"
 
 namespace sadmc {
+cudaError_t launch_lj_move_general(const MoveLaunch& m, const LjSys& s, int lpw, cudaStream_t st);
 cudaError_t launch_lj_move_sad(const MoveLaunch& m, const LjSys& s, int lpw, cudaStream_t st);
 namespace dev {
 
@@ -51,6 +52,7 @@ __global__ void lj_plan_kernel(WalkerCore* cores, LjSys s, int w, int which, flo
 
 cudaError_t launch_lj_move(const MoveLaunch& m, const LjSys& s, int lpw, cudaStream_t st) {
   if (m.method == M_SAD && !m.descent) return launch_lj_move_sad(m, s, lpw, st);
+  if (general_method(m.method) && !m.descent) return launch_lj_move_general(m, s, lpw, st);
   if (m.descent) {
     SADMC_LJ_ALL_SHAPES(dev::FAM_ANY, true)
   } else {

@@ -258,10 +258,11 @@ cudaError_t launch_lane(const MoveLaunch& m, const LjSys& s, cudaStream_t st) {
 bool lj_lane_shape(int lpw, int np) { return (lpw == 1 || lpw == 2) && (np == 32 || np == 64); }
 
 cudaError_t launch_lj_lane(const MoveLaunch& m, const LjSys& s, int lpw, cudaStream_t st) {
-  const bool sad = m.method == M_SAD;
 #define SADMC_LANE_CASE(L, N)                                                                  \
   if (lpw == L && s.np == N)                                                                   \
-    return sad ? dev::launch_lane<L, N, M_SAD>(m, s, st) : dev::launch_lane<L, N, dev::FAM_ANY>(m, s, st);
+    return m.method == M_SAD           ? dev::launch_lane<L, N, M_SAD>(m, s, st)                 \
+           : general_method(m.method) ? dev::launch_lane<L, N, dev::FAM_GENERAL>(m, s, st)      \
+                                      : dev::launch_lane<L, N, dev::FAM_ANY>(m, s, st);
   SADMC_LANE_CASE(1, 32)
   SADMC_LANE_CASE(2, 32)
   SADMC_LANE_CASE(1, 64)
