@@ -767,6 +767,11 @@ struct Fh {
     }
     lean_a1();
   }
+  // The same after general moves that were not followed by lean_sync.
+  __device__ void lean_resync() {
+    lw_lo = lw_hi = -1;  // lwlo and lwhi were not kept up
+    lean_sync();
+  }
   // ln w truncated to binary32 for 0 and [2^-126, 2^127): (double's bits >> 29) with the
   // exponent rebased, a smaller value as 0; a negative, huge or NaN weight gives NaN, which
   // leaves the Metropolis test undecided.
@@ -1247,6 +1252,24 @@ struct RecentScale {
     const int src = (int)off++;
     r = __shfl_sync(0xffffffffu, rs, src);
     om = __shfl_sync(0xffffffffu, omrs, src);
+  }
+};
+
+// Whether the walkers of a warp try the lean path.  They advance in step, so that a step costs
+// both paths if one of up to 32 walkers is on the general one: where that is most steps (fresh
+// walkers that discover their bins, energies on the bin edges, a method without a lean
+// path), the general path alone is quicker.  After 32 moves with kOften general ones among the
+// warp's walkers, all take it for kStretch times 32 moves; then the lean path is tried again.
+struct LeanTrial {
+  static constexpr uint32_t kOften = 20, kStretch = 15;
+  uint32_t general = 0, skip = 0;  // this walker's general moves; blocks of 32 still to skip
+  // Between blocks of 32 moves, by the whole warp; true: lean_resync is due.
+  __device__ bool next() {
+    bool again = false;
+    if (skip > 0) again = --skip == 0;
+    else if (__reduce_add_sync(0xffffffffu, general) >= kOften) skip = kStretch;
+    general = 0;
+    return again;
   }
 };
 
