@@ -240,21 +240,6 @@ struct CellOps {
     }
   }
 
-  // Sum over the candidates of one bucket k0 (0..26) around cell (cx,cy,cz) of query q
-  // (excluding atom `skip`); one lane per bucket.
-  __device__ static void scan(const CellWalker& cw, int k0, int cx, int cy, int cz, const Query& q,
-                              int skip, double wsqr, float wsqr32, bool newq, int& contacts,
-                              bool& overlap, float& e32) {
-    int ox, oy, oz;
-    const int c = bucket(cw, k0, cx, cy, cz, ox, oy, oz);
-    const int m = min(cw.cnt[c], cw.bucket);
-    const int* list = cw.atoms + (size_t)c * cw.bucket;
-    for (int k = 0; k < m; ++k) {
-      const int j = list[k];
-      if (j != skip) pair(cw, j, ox, oy, oz, q, wsqr, wsqr32, newq, contacts, overlap, e32);
-    }
-  }
-
   // The candidates of nq queries (1 or 2), 27 buckets each, spread evenly over the group:
   // query 0's buckets around (c0x, c0y, c0z) are entries 0..26 of bs, query 1's around
   // (c1x, c1y, c1z) entries 27..53.  Results go to each query's accumulators (SW:

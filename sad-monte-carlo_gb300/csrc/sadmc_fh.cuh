@@ -201,8 +201,8 @@ struct Fh {
   int win_lo, win_hi;  // SAD window as bin indices
   // gamma batch (see gamma())
   double gb_val[4];
-  uint32_t gb_base;  // low 32 bits of the move count the batch starts at
-  uint32_t gb_ok;    // bit q: gb_val[q] holds gamma for the current parameters
+  uint32_t gb_base;  // low 32 bits of the move count the batch starts at (one lane per walker)
+  uint32_t gb_ok;    // bit q: slot q holds gamma for the current parameters
   // per-move scratch
   double e1;
   int i2;
@@ -428,14 +428,14 @@ struct Fh {
       default: return 0.0;
     }
   }
-  // gamma(base + glane + LPW*q) sits in gb_val[q], base = the move count rounded down to a
-  // multiple of 4*LPW: four independent divide chains per lane hide the FP64 divide
-  // latency and cover 4*LPW moves.  The walkers of a launch share the move count, so the
-  // lane groups of a warp take their full refreshes at the same moves (one instruction
-  // stream).  A change of the SAD parameters mid-batch (gb_ok = 0) refreshes only the
-  // slot of the current move, one chain per lane for the next LPW moves, where other
-  // walkers share the warp.  (The low 32
-  // bits of the count suffice: a batch is replaced at least every 4*LPW moves.)
+  // Gamma of the 4 LPW moves from the move count rounded down to a multiple of that: four
+  // independent divide chains per lane hide the FP64 divide latency.  They sit in gtab, entry
+  // glane + LPW q from lane glane, or with one lane per walker in gb_val.  The walkers of a
+  // launch share the move count, so the lane groups of a warp take their full refreshes at
+  // the same moves (one instruction stream).  A change of the SAD parameters mid-batch (gb_ok = 0)
+  // refreshes only the slot of the current move, one chain per lane for the next LPW moves,
+  // where other walkers share the warp.  (The low 32 bits of the count suffice: a batch is
+  // replaced at least every 4 LPW moves.)
   // tF_d, ns_d, their reciprocals and g_zero for the current SAD parameters
   __device__ void refresh_sad_params() {
     if (c.tF != inv_tF_of) { tF_d = u2d(c.tF); inv_tF = 1.0 / tF_d; inv_tF_of = c.tF; }
@@ -450,15 +450,16 @@ struct Fh {
       if (kind() == M_SAD) refresh_sad_params();
       return gamma_at(c.moves);
     }
-    constexpr uint32_t SPAN = 4 * LPW;
-    if (LEAN && LPW > 1) {  // the batch in shared memory: one load per move
-      const int off = (int)((uint32_t)c.moves & (SPAN - 1)), qc = off / LPW;
+    if constexpr (LPW > 1) {
+      const int off = (int)((uint32_t)c.moves & (4u * LPW - 1)), qc = off / LPW;
       if (off == 0) gb_ok = 0;
       if (SADMC_RARE(!((gb_ok >> qc) & 1u))) {
         if (kind() == M_SAD) refresh_sad_params();
         const uint64_t t0 = c.moves - (uint64_t)off + (uint64_t)glane;
         sync();
         if (off == 0 || LPW == 32) {
+          // the batch boundary, or a warp that holds one walker (its chains run in parallel,
+          // so the remaining slots cost no more latency than one): every slot still ahead
 #pragma unroll
           for (int q = 0; q < 4; ++q)
             if (q >= qc) gtab[LPW * q + glane] = gamma_at(t0 + (uint64_t)(LPW * q));
@@ -470,37 +471,29 @@ struct Fh {
         sync();
       }
       return gtab[off];
-    }
-    const uint32_t m32 = (uint32_t)c.moves;
-    const uint32_t base = m32 & ~(SPAN - 1);
-    const int off = (int)(m32 - base);
-    const int qc = off / LPW;
-    if (base != gb_base) {
-      gb_base = base;
-      gb_ok = 0;
-    }
-    if (SADMC_RARE(!((gb_ok >> qc) & 1u))) {
-      if (kind() == M_SAD) refresh_sad_params();
-      const uint64_t t0 = c.moves - (uint64_t)off;
-      if (off == 0 || LPW == 32) {
-        // the batch boundary, or a warp that holds one walker (its chains run in parallel,
-        // so the remaining slots cost no more latency than one): every slot still ahead
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (q >= qc) gb_val[q] = gamma_at(t0 + (uint64_t)(glane + LPW * q));
-        gb_ok = 0xfu;
-      } else {
-        const double v = gamma_at(t0 + (uint64_t)(glane + LPW * qc));
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (q == qc) gb_val[q] = v;
-        gb_ok |= 1u << qc;
+    } else {
+      const uint32_t m32 = (uint32_t)c.moves, base = m32 & ~3u;
+      const int qc = (int)(m32 - base);
+      if (base != gb_base) {
+        gb_base = base;
+        gb_ok = 0;
       }
+      if (SADMC_RARE(!((gb_ok >> qc) & 1u))) {
+        if (kind() == M_SAD) refresh_sad_params();
+        if (qc == 0) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) gb_val[q] = gamma_at(c.moves + (uint64_t)q);
+          gb_ok = 0xfu;
+        } else {
+          const double v = gamma_at(c.moves);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (q == qc) gb_val[q] = v;
+          gb_ok |= 1u << qc;
+        }
+      }
+      return qc == 0 ? gb_val[0] : qc == 1 ? gb_val[1] : qc == 2 ? gb_val[2] : gb_val[3];
     }
-    const int q = off / LPW;
-    double v = q == 0 ? gb_val[0] : q == 1 ? gb_val[1] : q == 2 ? gb_val[2] : gb_val[3];
-    if (LPW == 1) return v;
-    return __shfl_sync(gmask, v, off % LPW, LPW);
   }
 
   // ---- have_visited_since_maxentropy as generation stamps ------------------------------
