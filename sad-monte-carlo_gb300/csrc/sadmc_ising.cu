@@ -20,9 +20,10 @@
 namespace sadmc {
 namespace dev {
 
-template <int LPW, int FAM, bool TRIAL>
+// TRIAL: the warp's walkers try the lean path as LeanTrial says.
 // (Two blocks to an SM: left to itself the compiler keeps to the 168 registers of three, 4096
 // walkers of 32 x 32, 8192 moves, 19.6 against 19.1 ms.)
+template <int LPW, int FAM, bool TRIAL>
 __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingSys s) {
   const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   const int lane = threadIdx.x & 31;

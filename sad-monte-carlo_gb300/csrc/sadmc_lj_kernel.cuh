@@ -103,9 +103,9 @@ struct LjWarpShared {
   double gamma[128];        // [walker][4 LPW]
 };
 
-template <int LPW, int APL, int FAM>
 // (Two blocks to an SM: left to itself the compiler may keep to the 168 registers of three and
 // spill, 4096 walkers of 31 atoms, 24414 moves, 57 against 47 ms.)
+template <int LPW, int APL, int FAM>
 __global__ void __launch_bounds__(128, 2) lj_move_kernel(MoveLaunch m, LjSys s) {
   const int wpw = LPW == 32 ? 1 : m.walkers_per_warp;
   __shared__ LjWarpShared<LPW, APL> sh[4];
