@@ -480,12 +480,13 @@ struct Fh {
       }
       if (SADMC_RARE(!((gb_ok >> qc) & 1u))) {
         if (kind() == M_SAD) refresh_sad_params();
+        const uint64_t t0 = c.moves - (uint64_t)qc;
         if (qc == 0) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) gb_val[q] = gamma_at(c.moves + (uint64_t)q);
+          for (int q = 0; q < 4; ++q) gb_val[q] = gamma_at(t0 + (uint64_t)q);
           gb_ok = 0xfu;
         } else {
-          const double v = gamma_at(c.moves);
+          const double v = gamma_at(t0 + (uint64_t)qc);
 #pragma unroll
           for (int q = 0; q < 4; ++q)
             if (q == qc) gb_val[q] = v;
