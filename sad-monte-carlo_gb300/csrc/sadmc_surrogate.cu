@@ -792,12 +792,15 @@ __global__ void take_flag_kernel(unsigned int* flag, unsigned int* out) { *out =
 
 cudaError_t sg_descriptors(const float* pos, int n, int configs, __nv_bfloat16* gq, cudaStream_t st) {
   using namespace dev;
-  // a warp per configuration from where the two kernels cross (38 atoms: 2048 configurations 36
-  // against 35 us, 4096 55 against 65; 13 atoms: 9.2 each, 11.8 against 13.9), while a block's
-  // shared memory stays below 48 KB
+  // A warp per configuration from where the two kernels cross, while a block's shared memory stays
+  // below 48 KB.  Up to 42 atoms six blocks share an SM and the crossing is near 2560 configurations
+  // (whole predictions: 42 atoms, 2560 configurations 98 us either way, 8192 228 against 200; 13
+  // atoms 49 against 47, 74 against 69); with fewer blocks the last wave weighs more, and it is near
+  // 6000 (44 atoms, 3072 configurations 112 against 132 us, 8192 233 against 219; 50 atoms, 2560
+  // configurations 117 against 148, 8192 284 either way).
   const int half = (n + 1) / 2;
   const size_t smem = sizeof(float2) * DESC_WARPS * (half * 32 + pair_rows(half));
-  if (configs >= 2560 && smem <= 48 * 1024) {
+  if (configs >= (smem <= 36 * 1024 ? 2560 : 6144) && smem <= 48 * 1024) {
     descriptor_pair_kernel<<<(configs + DESC_WARPS - 1) / DESC_WARPS, 32 * DESC_WARPS, smem, st>>>(pos, n, configs, gq);
   } else {
     const long long warps = (long long)configs * ((n + DESC_RPW - 1) / DESC_RPW);
