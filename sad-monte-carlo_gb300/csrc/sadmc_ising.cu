@@ -31,16 +31,20 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
   if (warp * wpw >= m.n_walkers) return;
   const int group = lane / LPW, glane = lane % LPW;
   const int w = warp * wpw + group;
-  // a lane past the warp's walkers touches no walker's memory: it leaves the descent, and fills
-  // the rate table with the others between the moves
+  // A lane past the warp's walkers touches no walker's memory.  It leaves the descent and a warp on
+  // trial (full, or the batch's last one), and else fills the rate table with the others between the
+  // moves: its FP64 chains are long for few lanes (64 walkers of 32 x 32, 8192 moves, 17.5 against
+  // 13.1 ms).  The branch around such lanes in the loop keeps its code off the uniform datapath,
+  // five branches a step more; a loop of their own for them was slower still (4096 walkers 16.8
+  // against 17.1 ms), an empty walker in each was quicker for SAD alone (16.3; SAMC 16.5 against 12.4).
   const bool own = group < wpw && w < m.n_walkers;
-  if (m.descent && !own) return;
+  if ((TRIAL || m.descent) && !own) return;
   const unsigned gmask = group_mask<LPW>(group);
   __shared__ RateTable rates[4];
   __shared__ double gammas[4][LPW > 1 ? 128 : 1];
   Fh<LPW, FAM, BOOK_LEAN, true> fh;
   const uint64_t moves0 = m.cores[warp * wpw].moves;  // the walkers share it
-  if (own) fh.load(m.cores, m.P, m.B, w, gmask, glane, true);
+  if (TRIAL || own) fh.load(m.cores, m.P, m.B, w, gmask, glane, true);
   const int L = s.L;
   int8_t* S = s.spins + (size_t)w * (size_t)L * (size_t)L;
   if (m.descent) {
@@ -78,7 +82,7 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
   RateTable& rt = rates[threadIdx.x >> 5];
   DrawCache<LPW, true> dc;
   dc.init();
-  if (own) {
+  if (TRIAL || own) {
     fh.gtab = gammas[threadIdx.x >> 5] + (LPW > 1 ? group * 4 * LPW : 0);
     fh.lean_sync();
   }
@@ -86,10 +90,11 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
   const uint32_t n_moves = (uint32_t)m.n_moves;
   for (uint32_t it = 0; it < n_moves; ++it) {
     if (SADMC_RARE((it & 31u) == 0)) {
-      rt.fill<1>(moves0 + it, lane, 32);
-      if (TRIAL && trial.next() && own) fh.lean_resync();
+      if (TRIAL) rt.fill<2>(moves0 + it, lane, warp_walkers(m.n_walkers, warp, wpw));
+      else rt.fill<1>(moves0 + it, lane, 32);
+      if (TRIAL && trial.next()) fh.lean_resync();
     }
-    if (!own) continue;
+    if (!TRIAL && !own) continue;
     const uint64_t t = fh.c.moves + 1;
     const double2 rate = rt.v[it & 31u];
     fh.begin_move(rate.y);
@@ -127,7 +132,7 @@ __global__ void __launch_bounds__(128, 2) ising_move_kernel(MoveLaunch m, IsingS
       if (LPW > 1) __syncwarp(gmask);
     }
   }
-  if (own) fh.store(m.cores, w);
+  if (TRIAL || own) fh.store(m.cores, w);
 }
 
 // compute_energy (ising.rs:59-75): sum over sites of s * (s_down + s_right), exact.

@@ -66,7 +66,7 @@ def test_one_lane_group_to_a_walker(name, function):
     assert "n_walkers - 1" not in body
     load = re.search(r"\w\.load\(m|= m\.cores\[w\]", body).start()
     assert re.search(r"if \(group >= wpw \|\| w >= m\.n_walkers\) return;", body[:load]) or re.search(
-        r"own = group < wpw && w < m\.n_walkers;.*if \(m\.descent && !own\) return;.*if \(own\) f$", body[:load], re.S)
+        r"own = group < wpw && w < m\.n_walkers;.*if \(\(TRIAL \|\| m\.descent\) && !own\) return;.*if \(TRIAL \|\| own\) f$", body[:load], re.S)
 
 
 @pytest.mark.parametrize("name", ["sadmc_fh.cuh", "sadmc_grand_book.cuh"])
