@@ -128,7 +128,7 @@ __global__ void cell_energy_kernel(const WalkerCore* cores, CellSys s, int n_wal
 // the axes run on three lanes, a bucket is one word, and a translation's two positions share
 // one query when they share a subcell; an ordinary SAMC move takes the lean path.
 // Bound by the chain of a step's dependent instructions and loads, with one warp per scheduler:
-// 512 walkers of up to 200 atoms, 4096 moves, 28.0 -> 14.4 ms.
+// 512 walkers of up to 200 atoms, 4096 moves, 28.0 -> 14.3 ms.
 template <int LPW>
 struct WcaGrandShared {
   float4 g[32];            // the normals and the atom pick (as int bits)

@@ -44,7 +44,7 @@ struct GrandWarpShared {
 // batch's moves (an add's position too), all kinds share one packed pair loop (an add has no
 // old position, a removal no new one), and an ordinary SAMC move takes the lean path.
 // Bound by the warp instructions of a step, with two warps per scheduler: 4096 walkers of up to
-// 31 atoms, 4096 moves, 20.9 -> 11.3 ms.  (Two blocks to an SM: left to itself the compiler keeps to
+// 31 atoms, 4096 moves, 20.9 -> 10.3 ms.  (Two blocks to an SM: left to itself the compiler keeps to
 // the 168 registers of three, 12.1 ms.)
 template <int LPW, int APL>
 __global__ void __launch_bounds__(128, 2) lj_grand_kernel(GrandLaunch m) {

@@ -1,8 +1,8 @@
 // 2D Ising model (src/system/ising.rs), many walkers per launch.
 //
 // An ordinary move takes the bookkeeping's lean path and sqrt(1/t) comes from a table in
-// shared memory: 4096 walkers of 32x32 run a step in 2.33 us instead of 4.55 (SAD; 3.30 with 32
-// walkers in a warp).
+// shared memory: 4096 walkers of 32x32 run a step in 2.45 us instead of 4.55 (SAD, eight to a
+// warp).
 //
 // Spins are int8 in global memory, index i + j*L (ising.rs:64).  A single-spin flip
 // changes E by -2 s_ij (sum of 4 periodic neighbours) (ising.rs:104-119); energies are

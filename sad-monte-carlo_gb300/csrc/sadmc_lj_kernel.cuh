@@ -15,8 +15,9 @@
 // per packed binary32 instruction (same roundings); draws, displacements, gamma and
 // sqrt(1/t) are tables in shared memory that all lanes fill, read back with one load each
 // instead of shuffles.  Measured on one GB300 (4096 LJ31 walkers, 8 lanes, SAD, past their
-// first 37 k moves): 990 -> 578 warp instructions per step, 3.53 -> 1.94 us; 1024 walkers
-// 3.17 -> 1.54 us (1.69 with four walkers in a warp).  The same walkers' first 12 k moves: 53.2 -> 37.8 ms.
+// first 37 k moves): 990 -> 592 warp instructions per step, 3.53 -> 1.77 us; 1024 walkers,
+// two in a warp, 3.17 -> 1.51 us.  The same 4096 walkers' first 24 k moves with copies and
+// descent: 98.7 -> 64.9 ms.
 //
 // Every resum_interval moves the energy
 // is replaced by an FP64 pair sum over the double-single positions (compute_energy,

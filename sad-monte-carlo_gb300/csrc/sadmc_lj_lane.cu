@@ -12,7 +12,7 @@
 // its atoms' values with one 64-bit load (conflict-free) for the packed pair terms, which
 // take two atoms per instruction.  Draws, gamma and sqrt(1/t) come from tables in shared
 // memory as in the register kernel.
-// Measured on one GB300 (8192 LJ38 walkers, 2 lanes, SAD): 8.8 -> 4.7 us per step against
+// Measured on one GB300 (8192 LJ38 walkers, 2 lanes, SAD): 8.8 -> 4.0 us per step against
 // the scalar pair terms over all 64 slots and the general bookkeeping on every move.
 // Global memory keeps the register kernel's [walker][6][np] planes, so the two kernels
 // continue each other's runs.
